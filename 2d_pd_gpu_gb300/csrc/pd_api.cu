@@ -269,6 +269,10 @@ Fp64Args fp64_args(pd_ctx* c) {
   a.inv_rho = 1.0 / c->p.rho;
   a.det_guard = c->p.det_guard;
   a.k_hg = c->p.k_hg;
+  a.k_hg2 = 2.0 * c->p.k_hg;
+  a.one = 1.0;
+  a.neg_one = -1.0;
+  a.neg_zero = -0.0;
   a.damage_fail = c->p.damage_fail;
   a.counters = c->counters;
   a.brk = c->p.s_c > 0.0;

@@ -32,6 +32,27 @@ __device__ __forceinline__ int64_t slot0(const Fp64Args& a, int64_t i, int* w) {
   return a.chunk_base[c] + (i & 31);
 }
 
+// Threads per block of the passes (32 particles): small blocks spread a small
+// plate over the chip (200 x 200, per step: 43 us against 47 with 128 threads
+// and 72 with 256) and end a large one evenly.
+constexpr int kPairBlock = 64;
+// Bonds in flight per thread (pass A 1, 2, 4: 22.6, 18.7, 19.0 us per step of
+// a 100 x 100 plate; pass B 2, 4: 21.6, 18.7).
+constexpr int kWalkA = 2, kWalkB = 4;
+
+// The passes run two threads per particle: thread h = 0 sums the x components
+// (d11, d12, the penalty's x; f.x), h = 1 the y components.  Every sum keeps
+// its operations and its order, none is computed twice, and each thread's
+// serial chain of FP64 operations is half as long: an FP64 instruction keeps
+// its SM quarter busy for 64 cycles, and that chain is what a plate too small
+// to fill the chip waits for.
+__device__ __forceinline__ double comp(const double2* p, int64_t i, int h) {
+  return reinterpret_cast<const double*>(p)[2 * i + h];
+}
+__device__ __forceinline__ void set_comp(double2* p, int64_t i, int h, double v) {
+  reinterpret_cast<double*>(p)[2 * i + h] = v;
+}
+
 // K^-1 and m/V of particle i over its intact bonds (oracle: kinv_of).
 __device__ void kinv_update(const Fp64Args& a, int64_t i) {
   int w;
@@ -67,6 +88,83 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
   const double rv = 1.0 / a.vol[i];
   a.mt[i] = make_double2(mx * rv, my * rv);
   a.singular[i] = 0;
+}
+
+// Pass A's update of the particles that lost bonds (newly > 0 in their lane):
+// broken count, damage, K^-1 and m/V, by the whole warp.  Eight lanes take a
+// particle, four particles at a time: lanes 0 .. 4 each sum one of k11, k12,
+// k22, mx, my in family order, lanes 0 .. 2 share one division (1 / det,
+// 1 / V, damage) and lanes 0 .. 4 one product; kinv_update's operations
+// (x + t is fma(t, 1, x)).  One thread alone has a chain of ~240 dependent FP64
+// operations here instead of ~45, each of which waits for its turn on the pipe,
+// and its pass waits for it (300 x 300 plate with bonds breaking, pass A:
+// 87 us against 72).
+__device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int64_t s0, int w, int newly) {
+  const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
+  unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
+  while (todo) {
+    unsigned rest = todo;  // this lane's particle: that of the (lane / 8)-th lane left to do
+    for (int q = lane >> 3; q > 0; --q) rest &= rest - 1;
+    const bool have = rest != 0;
+    const int src = have ? __ffs((int)rest) - 1 : 0;
+    const int64_t gi = __shfl_sync(0xffffffffu, i, src), gs = __shfl_sync(0xffffffffu, s0, src);
+    const int gw = __shfl_sync(0xffffffffu, w, src), gn = __shfl_sync(0xffffffffu, newly, src);
+    double sum = 0.0, num = 1.0, den = 1.0;
+    int nal = 0, broken = 0, fam = 1;
+    if (have) {
+      broken = a.broken[gi] + gn;
+      fam = a.fam[gi];
+      if (c == 1) den = a.vol[gi];
+      if (c == 2) {
+        num = (double)broken;
+        den = (double)fam;
+      }
+      const double* P = reinterpret_cast<const double*>(a.bgeo) + (c == 2 || c == 4 ? 1 : 0);  // V_j xi
+      const double* Q = reinterpret_cast<const double*>(a.bxi) + (c == 0 ? 0 : 1);             // xi
+      if (c < 5) {
+#pragma unroll 4
+        for (int k = 0; k < gw; ++k) {
+          const int64_t s = gs + (int64_t)k * kChunk;
+          const bool live = a.nbr[s] >= 0;
+          const double p = P[2 * s], q = c < 3 ? Q[2 * s] : 1.0;
+          if (live) {
+            sum = fma(p, q, sum);
+            ++nal;
+          }
+        }
+      }
+    }
+    const double k11 = __shfl_sync(0xffffffffu, sum, g0), k12 = __shfl_sync(0xffffffffu, sum, g0 + 1),
+                 k22 = __shfl_sync(0xffffffffu, sum, g0 + 2);
+    nal = __shfl_sync(0xffffffffu, nal, g0);
+    const double det = fma(k11, k22, -(k12 * k12));
+    if (c == 0) den = det;
+    const double quo = num / den;
+    const double r = __shfl_sync(0xffffffffu, quo, g0), rv = __shfl_sync(0xffffffffu, quo, g0 + 1),
+                 damage = __shfl_sync(0xffffffffu, quo, g0 + 2);
+    const bool bad = nal == 0 || damage > a.damage_fail || !(det > a.det_guard * (k11 * k22));
+    if (have) {
+      const double x = c == 0 ? k22 : c == 1 ? -k12 : c == 2 ? k11 : sum;
+      const double out = bad ? 0.0 : x * (c < 3 ? r : rv);
+      if (c < 2)
+        set_comp(a.kinv01, gi, c, out);
+      else if (c == 2)
+        a.kinv22[gi] = out;
+      else if (c < 5)
+        set_comp(a.mt, gi, c - 3, out);
+      else if (c == 5)
+        a.singular[gi] = bad ? 1 : 0;
+      else if (c == 6) {
+        a.broken[gi] = broken;
+        a.damage[gi] = damage;
+      } else {
+        atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)gn);
+        if (bad) atomicAdd(a.counters + CNT_SINGULAR, 1ull);
+      }
+    }
+    for (int q = 0; q < 4 && todo; ++q) todo &= todo - 1;
+  }
+  __syncwarp();  // the stores above are read by the particles' own lanes
 }
 
 __global__ void __launch_bounds__(kBlock) k_init_geometry(Fp64Args a) {
@@ -128,167 +226,222 @@ __device__ __forceinline__ bool surely_intact(float2 ui, float2 uj, float r2) {
   return fmaf(bx, bx, by * by) * 1.000001f <= r2;
 }
 
-// Pass A of particle i (stretch tests, D, penalty sum, stress, W).
+// Additions and products as fma, with the constant in a register: on this GPU a
+// DFMA of three registers leaves the FP64 pipe in 16 cycles per warp and SM; a
+// DADD, a DMUL, or a DFMA with an operand from the arguments or an immediate,
+// in 19 (measured, 4 to 16 warps).  x + y = fma(x, 1, y) and x y = fma(x, y, -0)
+// round the same exact value once and keep the sign of a zero.
+struct FpConst {
+  double one, neg_one, neg_zero;
+};
+// A value the compiler cannot place in a uniform register or fold (all lanes call it).
+__device__ __forceinline__ double in_register(double x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ FpConst fp_const(const Fp64Args& a) {
+  return FpConst{in_register(a.one), in_register(a.neg_one), in_register(a.neg_zero)};
+}
+__device__ __forceinline__ double add1(const FpConst& a, double x, double y) { return fma(x, a.one, y); }
+__device__ __forceinline__ double sub1(const FpConst& a, double x, double y) { return fma(y, a.neg_one, x); }
+__device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { return fma(x, y, a.neg_zero); }
+
+// Pass A of component h of particle i (stretch tests, D, penalty sum, stress,
+// W).  All 32 lanes of the warp call it, lanes 2k and 2k + 1 with the same
+// particle; ok = false: the lane has none.
+// Bonds are taken kWalkA at a time: the group's bond data and its neighbours'
+// state are requested together, and the next group's indices with them, so a
+// group costs one memory latency.
 template <bool BREAK, bool HG>
-__device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i) {
-  int w;
-  const int64_t s0 = slot0(a, i, &w);
-  const double2 ui = a.u[i];
-  const float2 ui32 = a.u32[i];
-  double d11 = 0.0, d12 = 0.0, d21 = 0.0, d22 = 0.0, ax = 0.0, ay = 0.0;
+__device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, int h, bool ok) {
+  int w = 0;
+  int64_t s0 = 0;
+  double ui = 0.0;
+  float2 ui32 = make_float2(0.f, 0.f);
+  if (ok) {
+    s0 = slot0(a, i, &w);
+    ui = comp(a.u, i, h);
+    if (BREAK) ui32 = a.u32[i];
+  }
+  const FpConst K = fp_const(a);
+  double d1 = 0.0, d2 = 0.0, ah = 0.0;  // row h of D, component h of the penalty sum
   int newly = 0;
-  for (int k = 0; k < w; ++k) {
+  int jn[kWalkA];
+#pragma unroll
+  for (int q = 0; q < kWalkA; ++q) jn[q] = q < w ? a.nbr[s0 + (int64_t)q * kChunk] : -1;
+  for (int k = 0; k < w; k += kWalkA) {
     const int64_t s = s0 + (int64_t)k * kChunk;
-    const int j = a.nbr[s];
-    if (j < 0) continue;
-    const double2 uj = a.u[j];
-    const double dx = uj.x - ui.x, dy = uj.y - ui.y;
-    if (BREAK && !surely_intact(ui32, a.u32[j], __ldcs(&a.br2[s]))) {
-      const double2 e = __ldcs(&a.bxi[s]);
-      const double q = fma(dx, fma(2.0, e.x, dx), dy * fma(2.0, e.y, dy));
-      if (q > __ldcs(&a.blim[s])) {
-        a.nbr[s] = -2 - j;
-        ++newly;
-        continue;
+    int j[kWalkA];
+    double uj[kWalkA], vj[kWalkA];
+    double2 t[kWalkA];
+    float2 uj32[kWalkA];
+    float r2[kWalkA];
+#pragma unroll
+    for (int q = 0; q < kWalkA; ++q) {
+      j[q] = jn[q];
+      const int64_t jj = j[q] < 0 ? i : (int64_t)j[q];  // (an empty slot reads the particle itself)
+      const int64_t sq = j[q] < 0 ? s : s + (int64_t)q * kChunk;
+      uj[q] = comp(a.u, jj, h);
+      t[q] = __ldcs(&a.bgeo[sq]);
+      if (HG) vj[q] = a.vol[jj];
+      if (BREAK) {
+        uj32[q] = a.u32[jj];
+        r2[q] = __ldcs(&a.br2[sq]);
       }
     }
-    const double2 t = __ldcs(&a.bgeo[s]);
-    d11 = fma(dx, t.x, d11);
-    d12 = fma(dx, t.y, d12);
-    d21 = fma(dy, t.x, d21);
-    d22 = fma(dy, t.y, d22);
-    if (HG) {
-      const double vj = a.vol[j];
-      ax = fma(vj, dx, ax);
-      ay = fma(vj, dy, ay);
+#pragma unroll
+    for (int q = 0; q < kWalkA; ++q)
+      jn[q] = k + kWalkA + q < w ? a.nbr[s + (int64_t)(kWalkA + q) * kChunk] : -1;
+#pragma unroll
+    for (int q = 0; q < kWalkA; ++q) {
+      if (j[q] < 0) continue;
+      if (BREAK && !surely_intact(ui32, uj32[q], r2[q])) {
+        const int64_t sq = s + (int64_t)q * kChunk;
+        const double2 e = __ldcs(&a.bxi[sq]), ua = a.u[i], ub = a.u[j[q]];
+        const double dx = ub.x - ua.x, dy = ub.y - ua.y;
+        const double z = fma(dx, fma(2.0, e.x, dx), dy * fma(2.0, e.y, dy));
+        if (z > __ldcs(&a.blim[sq])) {
+          // both threads of the pair find the same; the second one does not store, and if it
+          // reads the slot after the first one's store it skips the bond there
+          if (h == 0) a.nbr[sq] = -2 - j[q];
+          ++newly;
+          continue;
+        }
+      }
+      const double dh = sub1(K, uj[q], ui);
+      d1 = fma(dh, t[q].x, d1);
+      d2 = fma(dh, t[q].y, d2);
+      if (HG) ah = fma(vj[q], dh, ah);
     }
   }
-  if (HG) {
-    const double k2 = 2.0 * a.k_hg;
-    a.hg[i] = make_double2(k2 * ax, k2 * ay);
+  // late, so that the next pass's blocks do not take the places of this pass's waiting ones
+  grid_dep_launch();
+  if (HG && ok) set_comp(a.hg, i, h, mul1(K, a.k_hg2, ah));
+  if (BREAK) {
+    newly = __shfl_sync(0xffffffffu, newly, threadIdx.x & 30);  // the first thread's count
+    if (__any_sync(0xffffffffu, newly != 0)) kinv_update_warp(a, i, s0, w, h == 0 ? newly : 0);
   }
-  if (BREAK && newly) {
-    atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)newly);
-    const int32_t b = a.broken[i] + newly;
-    a.broken[i] = b;
-    a.damage[i] = (double)b / (double)a.fam[i];
-    kinv_update(a, i);
+  double2 k01 = make_double2(0.0, 0.0);
+  double k22 = 0.0, vi = 0.0;
+  bool singular = true;
+  if (ok) {
+    singular = a.singular[i];
+    k01 = a.kinv01[i];
+    k22 = a.kinv22[i];
+    vi = a.vol[i];
   }
-  if (a.singular[i]) {
-    a.w01[i] = make_double2(0.0, 0.0);
-    a.w23[i] = make_double2(0.0, 0.0);
-    return;
-  }
-  const double2 k01 = a.kinv01[i];
-  const double k11 = k01.x, k12 = k01.y, k22 = a.kinv22[i];
-  // G = D K^-1 = F - I
-  const double g11 = fma(d11, k11, d12 * k12), g12 = fma(d11, k12, d12 * k22);
-  const double g21 = fma(d21, k11, d22 * k12), g22 = fma(d21, k12, d22 * k22);
-  const double e11 = g11, e22 = g22, e12 = 0.5 * (g12 + g21);
-  const double s11 = fma(a.c11, e11, a.c12 * e22);
-  const double s22 = fma(a.c12, e11, a.c11 * e22);
-  const double s12 = a.c33 * e12;
-  const double vi = a.vol[i];
+  const double k11 = k01.x, k12 = k01.y;
+  // row h of G = D K^-1 = F - I, and of the symmetric stress: thread 0 has
+  // (s11, s12), thread 1 (s12, s22)
+  const double g1 = fma(d1, k11, mul1(K, d2, k12)), g2 = fma(d1, k12, mul1(K, d2, k22));
+  const double diag = h ? g2 : g1, other = __shfl_xor_sync(0xffffffffu, diag, 1);
+  const double off = h ? g1 : g2, cross = __shfl_xor_sync(0xffffffffu, off, 1);
+  const double e11 = h ? other : diag, e22 = h ? diag : other, e12 = mul1(K, 0.5, add1(K, off, cross));
+  const double sd = fma(h ? a.c12 : a.c11, e11, mul1(K, h ? a.c11 : a.c12, e22));
+  const double s12 = mul1(K, a.c33, e12);
+  const double sa = h ? s12 : sd, sb = h ? sd : s12;
+  if (!ok) return;
+  double w1 = fma(sa, k11, mul1(K, sb, k12)), w2 = fma(sa, k12, mul1(K, sb, k22));
   if (HG) {  // W = V (sigma K^-1 - k G)
     const double kh = -a.k_hg;
-    a.w01[i] = make_double2(vi * fma(kh, g11, fma(s11, k11, s12 * k12)), vi * fma(kh, g12, fma(s11, k12, s12 * k22)));
-    a.w23[i] = make_double2(vi * fma(kh, g21, fma(s12, k11, s22 * k12)), vi * fma(kh, g22, fma(s12, k12, s22 * k22)));
-  } else {
-    a.w01[i] = make_double2(vi * fma(s11, k11, s12 * k12), vi * fma(s11, k12, s12 * k22));
-    a.w23[i] = make_double2(vi * fma(s12, k11, s22 * k12), vi * fma(s12, k12, s22 * k22));
+    w1 = fma(kh, g1, w1);
+    w2 = fma(kh, g2, w2);
   }
+  double2 W = make_double2(mul1(K, vi, w1), mul1(K, vi, w2));
+  if (singular) W = make_double2(0.0, 0.0);
+  (h ? a.w23 : a.w01)[i] = W;
 }
 
 template <bool BREAK, bool HG>
-__global__ void __launch_bounds__(kBlock) k_pass_a(Fp64Args a) {
-  const int64_t i = a.i0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  grid_dep_sync();  // nothing is read before the previous pass has completed
-  if (i < a.n) pass_a_particle<BREAK, HG>(a, i);
+__global__ void __launch_bounds__(kPairBlock) k_pass_a(Fp64Args a) {
+  const int64_t i = a.i0 + (int64_t)blockIdx.x * (kPairBlock / 2) + (threadIdx.x >> 1);
+  grid_dep_wait();  // nothing is read before the previous pass has completed
+  pass_a_particle<BREAK, HG>(a, i, threadIdx.x & 1, i < a.n);
 }
 
-// Pass B of particle i (force gather, kick; MODE 1 adds the next drift,
-// MODE 2 is the drop-in kick with acce in/out).
+// Pass B of component h of particle i (force gather, kick; MODE 1 adds the
+// next drift, MODE 2 is the drop-in kick with acce in/out).
 template <int MODE, bool HG>
-__device__ __forceinline__ void pass_b_particle(const Fp64Args& a, int64_t i) {
+__device__ __forceinline__ void pass_b_particle(const Fp64Args& a, const FpConst& K, int64_t i, int h) {
   int w;
   const int64_t s0 = slot0(a, i, &w);
-  const double2 wa = a.w01[i], wb = a.w23[i], m = a.mt[i];
-  double fx, fy;
-  if (HG) {
-    const double2 h = a.hg[i];
-    fx = fma(wa.x, m.x, fma(wa.y, m.y, h.x));
-    fy = fma(wb.x, m.x, fma(wb.y, m.y, h.y));
-  } else {
-    fx = fma(wa.x, m.x, wa.y * m.y);
-    fy = fma(wb.x, m.x, wb.y * m.y);
+  const double2* W = h ? a.w23 : a.w01;
+  const double2 wi = W[i], m = a.mt[i];
+  double f = fma(wi.x, m.x, HG ? fma(wi.y, m.y, comp(a.hg, i, h)) : mul1(K, wi.y, m.y));
+  // requested before the walk (1M-particle plate: 252 -> 243 us)
+  double v = comp(a.v, i, h), ao = comp(MODE == 2 ? a.acc : a.f, i, h), u = MODE == 1 ? comp(a.u, i, h) : 0.0;
+  int jn[kWalkB];
+#pragma unroll
+  for (int q = 0; q < kWalkB; ++q) jn[q] = q < w ? __ldcs(&a.nbr[s0 + (int64_t)q * kChunk]) : -1;
+  for (int k = 0; k < w; k += kWalkB) {  // as pass A's walk
+    const int64_t s = s0 + (int64_t)k * kChunk;
+    int j[kWalkB];
+    double2 nb[kWalkB], e[kWalkB];
+#pragma unroll
+    for (int q = 0; q < kWalkB; ++q) {
+      j[q] = jn[q];
+      nb[q] = W[j[q] < 0 ? i : (int64_t)j[q]];
+      e[q] = __ldcs(&a.bxi[j[q] < 0 ? s : s + (int64_t)q * kChunk]);
+    }
+#pragma unroll
+    for (int q = 0; q < kWalkB; ++q)
+      jn[q] = k + kWalkB + q < w ? __ldcs(&a.nbr[s + (int64_t)(kWalkB + q) * kChunk]) : -1;
+#pragma unroll
+    for (int q = 0; q < kWalkB; ++q) {
+      if (j[q] < 0) continue;
+      f = fma(nb[q].x, e[q].x, f);
+      f = fma(nb[q].y, e[q].y, f);
+    }
   }
-  struct Nb {
-    double2 a, b;
-  };
-  walk_bonds<4>(
-      w, i, GlobalIdx{a.nbr, s0}, [&](int64_t j) { return Nb{a.w01[j], a.w23[j]}; },
-      [&](int k, int, const Nb& nb) {
-        const double2 e = __ldcs(&a.bxi[s0 + (int64_t)k * kChunk]);
-        fx = fma(nb.a.x, e.x, fx);
-        fx = fma(nb.a.y, e.y, fx);
-        fy = fma(nb.b.x, e.x, fy);
-        fy = fma(nb.b.y, e.y, fy);
-      });
-  double2 v = a.v[i];
-  double aox, aoy;
-  if (MODE == 2) {
-    const double2 ao = a.acc[i];
-    aox = ao.x;
-    aoy = ao.y;
-  } else {
-    const double2 fo = a.f[i];
-    aox = fo.x * a.inv_rho;
-    aoy = fo.y * a.inv_rho;
+  grid_dep_launch();
+  if (MODE != 2) ao = mul1(K, ao, a.inv_rho);
+  const double an = mul1(K, f, a.inv_rho);
+  v = add1(K, v, mul1(K, mul1(K, 0.5, add1(K, ao, an)), a.dt));
+  set_comp(a.f, i, h, f);
+  if (MODE == 2) set_comp(a.acc, i, h, an);
+  if (MODE == 1) {  // drift_one of the component
+    const int g = a.bc[i];
+    const int kind = g ? a.gkind[g - 1] : PD_BC_NONE;
+    if (kind == PD_BC_VELOCITY) v = comp(a.gval, g - 1, h);
+    u = add1(K, u, add1(K, mul1(K, v, a.dt), mul1(K, mul1(K, 0.5, an), a.dt2)));
+    if (kind == PD_BC_FIXED) u = 0.0;
+    set_comp(a.u, i, h, u);
+    reinterpret_cast<float*>(a.u32)[2 * i + h] = (float)u;
   }
-  const double anx = fx * a.inv_rho, any = fy * a.inv_rho;
-  v.x = v.x + (0.5 * (aox + anx)) * a.dt;
-  v.y = v.y + (0.5 * (aoy + any)) * a.dt;
-  a.f[i] = make_double2(fx, fy);
-  if (MODE == 2) a.acc[i] = make_double2(anx, any);
-  if (MODE == 1) {
-    double2 u = a.u[i];
-    drift_one(a, i, v, u, anx, any);
-    a.u[i] = u;
-    a.u32[i] = make_float2((float)u.x, (float)u.y);
-  }
-  a.v[i] = v;
+  set_comp(a.v, i, h, v);
   if (a.out_v) {  // pd_step_host's last pass, or the drop-in call: the results straight to host memory
     if (MODE == 2)
-      a.out_a[i] = make_double2(anx, any);
+      set_comp(a.out_a, i, h, an);
     else
-      a.out_u[i] = a.u[i];
-    a.out_v[i] = v;
-    a.out_f[i] = make_double2(fx, fy);
+      set_comp(a.out_u, i, h, MODE == 1 ? u : comp(a.u, i, h));
+    set_comp(a.out_v, i, h, v);
+    set_comp(a.out_f, i, h, f);
   }
 }
 
 template <int MODE, bool HG>
-// 6 blocks per SM (<= 40 registers, no spills): 262 -> 258 us on the 1M-particle plate
-__global__ void __launch_bounds__(kBlock, 6) k_pass_b(Fp64Args a) {
-  const int64_t i = a.i0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  grid_dep_sync();
-  if (i < a.n) pass_b_particle<MODE, HG>(a, i);
+__global__ void __launch_bounds__(kPairBlock) k_pass_b(Fp64Args a) {
+  const int64_t i = a.i0 + (int64_t)blockIdx.x * (kPairBlock / 2) + (threadIdx.x >> 1);
+  grid_dep_wait();
+  const FpConst K = fp_const(a);
+  if (i < a.n) pass_b_particle<MODE, HG>(a, K, i, threadIdx.x & 1);
 }
 
 // ---- batched plates: phase 0 drift, 1 pass A, 2 pass B + next drift, 3 pass B
-__device__ __forceinline__ void batch_particle(const Fp64Args& p, int64_t i, int phase) {
+// (ok = false: a lane past the tile's end, which only the warp-wide parts call for)
+__device__ __forceinline__ void batch_particle(const Fp64Args& p, int64_t i, int h, bool ok, int phase) {
   const bool hg = p.k_hg != 0.0;
   if (phase == 0) {
-    drift_particle(p, i);
+    if (ok && h == 0) drift_particle(p, i);
   } else if (phase == 1) {
     if (p.brk)
-      hg ? pass_a_particle<true, true>(p, i) : pass_a_particle<true, false>(p, i);
+      hg ? pass_a_particle<true, true>(p, i, h, ok) : pass_a_particle<true, false>(p, i, h, ok);
     else
-      hg ? pass_a_particle<false, true>(p, i) : pass_a_particle<false, false>(p, i);
-  } else if (phase == 2) {
-    hg ? pass_b_particle<1, true>(p, i) : pass_b_particle<1, false>(p, i);
+      hg ? pass_a_particle<false, true>(p, i, h, ok) : pass_a_particle<false, false>(p, i, h, ok);
   } else {
-    hg ? pass_b_particle<0, true>(p, i) : pass_b_particle<0, false>(p, i);
+    const FpConst K = fp_const(p);
+    if (!ok) return;
+    if (phase == 2)
+      hg ? pass_b_particle<1, true>(p, K, i, h) : pass_b_particle<1, false>(p, K, i, h);
+    else
+      hg ? pass_b_particle<0, true>(p, K, i, h) : pass_b_particle<0, false>(p, K, i, h);
   }
 }
 
@@ -297,7 +450,10 @@ __device__ __forceinline__ void batch_phase(const Fp64Args* __restrict__ plates,
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BatchTile T = tiles[t];
     const Fp64Args& p = plates[T.plate];
-    for (int k = threadIdx.x; k < T.count; k += blockDim.x) batch_particle(p, T.first + k, phase);
+    for (int k0 = 0; k0 < 2 * T.count; k0 += blockDim.x) {  // whole warps in every round
+      const int k = k0 + threadIdx.x;
+      batch_particle(p, T.first + (k >> 1), k & 1, k < 2 * T.count, phase);
+    }
   }
 }
 
@@ -359,9 +515,6 @@ cudaError_t launch_batch_fp64(const Fp64Args* d_plates, const BatchTile* d_tiles
 }
 
 namespace {
-}  // namespace
-
-namespace {
 // reach[k] / low[k] = the largest / smallest id among slab k's particles
 // (k*slab .. k*slab + slab - 1) and their neighbours
 __global__ void k_slab_reach(int64_t n, const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
@@ -399,8 +552,8 @@ void launch_shadow_fp64(const Fp64Args& a, cudaStream_t s) {
 // while the previous kernel on the stream drains, and wait for it first).
 static void launch_pass(void (*kernel)(Fp64Args), const Fp64Args& a, bool pdl, cudaStream_t s) {
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3((unsigned)blocks_for(a.n - a.i0));
-  lc.blockDim = dim3(kBlock);
+  lc.gridDim = dim3((unsigned)blocks_for(2 * (a.n - a.i0), kPairBlock));
+  lc.blockDim = dim3(kPairBlock);
   lc.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -101,7 +101,8 @@ struct Fp64Args {
   double2* out_f;
   double2* out_a;
   double c11, c12, c33;
-  double dt, dt2, inv_rho, det_guard, k_hg, damage_fail;
+  double dt, dt2, inv_rho, det_guard, k_hg, k_hg2, damage_fail;  // k_hg2 = 2 k_hg
+  double one, neg_one, neg_zero;  // 1, -1, -0 (add1, sub1, mul1)
   unsigned long long* counters;
   int32_t brk;  // bond breaking on (s_c > 0)
   int32_t pad;

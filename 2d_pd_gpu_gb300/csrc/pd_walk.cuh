@@ -23,9 +23,11 @@ namespace pd {
 // serialization starts while the previous pass drains; grid_dep_sync() waits
 // until that pass has completed and its writes are visible, then lets the next
 // pass launch.  Without the launch attribute both instructions return at once.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_sync() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  grid_dep_wait();
+  grid_dep_launch();
 }
 
 template <int U, typename Idx, typename Gather, typename Body>
