@@ -52,8 +52,7 @@ struct pd_ctx {
   pd::SellLayout sell;
   pd::HaloLayout halo;  // mixed form
   double2 *bxi = nullptr, *bgeo = nullptr;
-  double* blim = nullptr;
-  float* br2 = nullptr;
+  float2* bxi32 = nullptr;
   float2* u32 = nullptr;
   // bond-associated mode
   double2* tb = nullptr;
@@ -187,8 +186,7 @@ void free_families(pd_ctx* c) {
   c->halo = pd::HaloLayout{};
   dfree(c->bxi);
   dfree(c->bgeo);
-  dfree(c->blim);
-  dfree(c->br2);
+  dfree(c->bxi32);
   dfree(c->tb);
   dfree(c->rslot);
   dfree(c->ba_lr);
@@ -262,7 +260,7 @@ Fp64Args fp64_args(pd_ctx* c) {
   a.bc = c->bc; a.gkind = c->gkind; a.gval = c->gval;
   a.broken = c->broken; a.damage = c->damage; a.singular = c->singular; a.fam = c->fam;
   a.chunk_base = c->sell.chunk_base; a.chunk_w = c->sell.chunk_w; a.nbr = c->sell.nbr;
-  a.bxi = c->bxi; a.bgeo = c->bgeo; a.blim = c->blim; a.br2 = c->br2; a.u32 = c->u32;
+  a.bxi = c->bxi; a.bgeo = c->bgeo; a.bxi32 = c->bxi32; a.u32 = c->u32;
   stiffness(c, &a.c11, &a.c12, &a.c33);  // getStiffnessTensor, src/main_seq.cpp:185-187
   a.dt = c->p.dt;
   a.dt2 = c->p.dt * c->p.dt;
@@ -273,6 +271,7 @@ Fp64Args fp64_args(pd_ctx* c) {
   a.one = 1.0;
   a.neg_one = -1.0;
   a.neg_zero = -0.0;
+  a.s2 = c->p.s_c > 0.0 ? c->p.s_c * (2.0 + c->p.s_c) : INFINITY;
   a.damage_fail = c->p.damage_fail;
   a.counters = c->counters;
   a.brk = c->p.s_c > 0.0;
@@ -445,10 +444,8 @@ int finish_families(pd_ctx* c) {
     const size_t ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
     PD_CK(c, cudaMalloc(&c->bxi, ns * sizeof(double2)));
     PD_CK(c, cudaMalloc(&c->bgeo, ns * sizeof(double2)));
-    PD_CK(c, cudaMalloc(&c->blim, ns * sizeof(double)));
-    PD_CK(c, cudaMalloc(&c->br2, ns * sizeof(float)));
-    pd::launch_bond_geometry_fp64(c->n, c->x, c->vol, c->sell, c->row_ptr, c->p.s_c, c->bxi, c->bgeo, c->blim,
-                                  c->br2, s);
+    PD_CK(c, cudaMalloc(&c->bxi32, ns * sizeof(float2)));
+    pd::launch_bond_geometry_fp64(c->n, c->x, c->vol, c->sell, c->bxi, c->bgeo, c->bxi32, s);
   } else {
     // mixed-form scales: Ls = the family cutoff (or the longest bond), Vs = mean volume
     double ls = c->cutoff;
@@ -587,7 +584,6 @@ int pd_set_params(pd_ctx* c, const pd_params* p) {
   if (p->device != c->p.device || p->precision != c->p.precision)
     return fail(c, PD_ERR_ARG, "device and precision are fixed at pd_create");
   PD_CK(c, cudaSetDevice(c->p.device));
-  const bool s_changed = p->s_c != c->p.s_c;
   c->p = *p;
   c->c_override = false;
   clear_graphs(c);
@@ -596,11 +592,6 @@ int pd_set_params(pd_ctx* c, const pd_params* p) {
     if (rc2 != PD_OK) return rc2;
     rc2 = ensure_ba(c);
     if (rc2 != PD_OK) return rc2;
-  }
-  if (c->has_families && s_changed && !mixed(c)) {
-    pd::launch_bond_limit_fp64(c->sell.nslots, c->bxi, c->p.s_c, c->sell.nbr, c->blim, c->br2, c->stream);
-    PD_CK(c, cudaGetLastError());
-    PD_CK(c, cudaStreamSynchronize(c->stream));
   }
   return PD_OK;
 }

@@ -268,19 +268,10 @@ __global__ void k_sell_fill(int64_t n, const int64_t* __restrict__ row_ptr, cons
   }
 }
 
-// Stretch limits of a bond: the exact FP64 one, and the FP32 certificate
-// threshold (s_c |xi|)^2 (1 - 1e-5) rounded toward zero (never above the truth).
-__device__ __forceinline__ void bond_limits(double ex, double ey, double s_c, double* lim, float* r2) {
-  const double ee = fma(ex, ex, ey * ey);
-  const double s2 = s_c > 0.0 ? s_c * (2.0 + s_c) : INFINITY;
-  *lim = s2 * ee;
-  *r2 = s_c > 0.0 ? __double2float_rz(((s_c * s_c) * ee) * (1.0 - 1e-5)) : 0.0f;
-}
-
 __global__ void k_bond_geometry(int64_t n, const double2* __restrict__ x, const double* __restrict__ vol,
                                 const int64_t* __restrict__ chunk_base, const int32_t* __restrict__ chunk_w,
-                                const int32_t* __restrict__ pos_of, const int32_t* __restrict__ nbr, double s_c,
-                                double2* bxi, double2* bgeo, double* blim, float* br2) {
+                                const int32_t* __restrict__ pos_of, const int32_t* __restrict__ nbr,
+                                double2* bxi, double2* bgeo, float2* bxi32) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t p = sell_pos(pos_of, i);
@@ -294,8 +285,7 @@ __global__ void k_bond_geometry(int64_t n, const double2* __restrict__ x, const 
     if (j < 0) {
       bxi[s] = make_double2(0.0, 0.0);
       bgeo[s] = make_double2(0.0, 0.0);
-      blim[s] = 0.0;
-      br2[s] = 0.0f;
+      bxi32[s] = make_float2(0.f, 0.f);
       continue;
     }
     const double2 pj = x[j];
@@ -303,20 +293,7 @@ __global__ void k_bond_geometry(int64_t n, const double2* __restrict__ x, const 
     const double vj = vol[j];
     bxi[s] = make_double2(ex, ey);
     bgeo[s] = make_double2(vj * ex, vj * ey);
-    bond_limits(ex, ey, s_c, &blim[s], &br2[s]);
-  }
-}
-
-__global__ void k_bond_limit(int64_t nslots, const double2* __restrict__ bxi, double s_c,
-                             const int32_t* __restrict__ nbr, double* blim, float* br2) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslots) return;
-  const double2 e = bxi[s];
-  if (nbr[s] == -1) {
-    blim[s] = 0.0;
-    br2[s] = 0.0f;
-  } else {
-    bond_limits(e.x, e.y, s_c, &blim[s], &br2[s]);
+    bxi32[s] = make_float2((float)ex, (float)ey);
   }
 }
 
@@ -505,16 +482,10 @@ int build_sell(int64_t n, const int64_t* d_row_ptr, const int32_t* d_col, cudaSt
 }
 
 void launch_bond_geometry_fp64(int64_t n, const double2* x, const double* vol, const SellLayout& L,
-                               const int64_t* /*row_ptr*/, double s_c, double2* bxi, double2* bgeo, double* blim,
-                               float* br2, cudaStream_t s) {
+                               double2* bxi, double2* bgeo, float2* bxi32, cudaStream_t s) {
   if (n > 0)
     k_bond_geometry<<<(unsigned)blocks_for(n), kBlock, 0, s>>>(n, x, vol, L.chunk_base, L.chunk_w, L.pos_of, L.nbr,
-                                                              s_c, bxi, bgeo, blim, br2);
-}
-
-void launch_bond_limit_fp64(int64_t nslots, const double2* bxi, double s_c, const int32_t* nbr, double* blim,
-                            float* br2, cudaStream_t s) {
-  if (nslots > 0) k_bond_limit<<<(unsigned)blocks_for(nslots), kBlock, 0, s>>>(nslots, bxi, s_c, nbr, blim, br2);
+                                                              bxi, bgeo, bxi32);
 }
 
 void launch_mask_out(int64_t n, const int64_t* row_ptr, const int32_t* col, const SellLayout& L, uint8_t* alive,

@@ -17,8 +17,8 @@
 //                           f_i = sum_j V_j (S_i + S_j) xi_ij (= T_ij - T_ji)
 // FP64 operations per bond: pass A 11 (d 2, stretch test 5, D 4) + 2 with the
 // zero-energy-mode penalty (sum V_j d), pass B 4.  The stretch test runs in
-// FP64 only for bonds an FP32 bound cannot prove intact (surely_intact), so
-// pass A costs 8 FP64 operations for almost every bond.
+// FP64 only for bonds within ~1e-6 of the limit (stretch_fp32 proves its
+// outcome for the others), so pass A costs 8 FP64 operations per bond.
 #include "pd_internal.h"
 #include "pd_walk.cuh"
 
@@ -212,18 +212,38 @@ __global__ void __launch_bounds__(kBlock) k_shadow(Fp64Args a) {
   a.u32[i] = make_float2((float)u.x, (float)u.y);
 }
 
-// FP32 certificate that a bond is intact: an upper bound B on the FP64
-// |d| = |fl64(u_j - u_i)| from the FP32 shadows (|u - fl32(u)| <= 2^-24 |u|,
-// FP32 rounding of the difference and of B itself covered by the 6e-8 and
-// 1.000001 factors) with B^2 <= (s_c |xi|)^2 (1 - 1e-5).  Then
-// d.(2 xi + d) <= 2|xi|B + B^2 < ((1 + s_c)^2 - 1)|xi|^2 by a relative
-// margin >= 5e-6, far above the FP64 evaluation error of the exact test, so
-// the FP64 test would say "intact": skipping it cannot change any result.
-__device__ __forceinline__ bool surely_intact(float2 ui, float2 uj, float r2) {
+// The stretch test in FP32 from the shadows of u and xi: 1 the FP64 test would
+// say intact, -1 it would say broken, 0 too close to call (the FP64 test runs).
+// With f = fl32(u32_j - u32_i), S_c = 2|xi_c| + |f_c| and delta_c a bound on
+// |f_c - d_c| (the shadows' and the difference's rounding, <= 2^-24 each of
+// |u_j|, |u_i| and |f|), the FP64 test's q = d.(2 xi + d) differs from
+// f.(2 xi + f) by at most sum delta_c (2 S_c + delta_c), and xi's and the
+// evaluation's rounding add at most 4 * 2^-24 sum |f_c| S_c; the limit's own
+// relative error is below 6 * 2^-24.  The margins taken (6.0e-8, 3e-7 and 1e-6)
+// are above these and the FP64 evaluation's ~1e-15.  Limits where FP32 products
+// could underflow or overflow, and any infinity or NaN, leave it to FP64.
+// A test that bounds |d| alone leaves every rotating or compressed bond to FP64
+// too, which in the few warps of a fracture zone is what the whole pass waits
+// for (300 x 300 plate with bonds breaking: see k_pass_a).
+__device__ __forceinline__ int stretch_fp32(float2 ui, float2 uj, float2 e, float s2) {
   const float fx = uj.x - ui.x, fy = uj.y - ui.y;
-  const float bx = fabsf(fx) + 6.0e-8f * (fabsf(uj.x) + fabsf(ui.x) + fabsf(fx));
-  const float by = fabsf(fy) + 6.0e-8f * (fabsf(uj.y) + fabsf(ui.y) + fabsf(fy));
-  return fmaf(bx, bx, by * by) * 1.000001f <= r2;
+  const float dx = 6.0e-8f * (fabsf(uj.x) + fabsf(ui.x) + fabsf(fx));
+  const float dy = 6.0e-8f * (fabsf(uj.y) + fabsf(ui.y) + fabsf(fy));
+  const float sx = fmaf(2.0f, fabsf(e.x), fabsf(fx)), sy = fmaf(2.0f, fabsf(e.y), fabsf(fy));
+  const float q = fmaf(fx, fmaf(2.0f, e.x, fx), fy * fmaf(2.0f, e.y, fy));
+  const float err = fmaf(3.0e-7f, fmaf(fabsf(fx), sx, fabsf(fy) * sy),
+                         fmaf(dx, fmaf(2.0f, sx, dx), dy * fmaf(2.0f, sy, dy)));
+  const float lim = s2 * fmaf(e.x, e.x, e.y * e.y);
+  if (!(lim > 1.0e-30f && lim < 1.0e30f)) return 0;
+  if (q + err < 0.999999f * lim) return 1;
+  return q - err > 1.000001f * lim ? -1 : 0;
+}
+
+// The same in FP64 (the oracle's operations).
+__device__ __noinline__ bool stretch_fp64(const Fp64Args& a, int64_t i, int64_t j, int64_t s) {
+  const double2 e = a.bxi[s], ui = a.u[i], uj = a.u[j];
+  const double dx = uj.x - ui.x, dy = uj.y - ui.y;
+  return fma(dx, fma(2.0, e.x, dx), dy * fma(2.0, e.y, dy)) > a.s2 * fma(e.x, e.x, e.y * e.y);
 }
 
 // Additions and products as fma, with the constant in a register: on this GPU a
@@ -263,6 +283,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   const FpConst K = fp_const(a);
   double d1 = 0.0, d2 = 0.0, ah = 0.0;  // row h of D, component h of the penalty sum
   int newly = 0;
+  const float s2 = BREAK ? (float)a.s2 : 0.f;
   int jn[kWalkA];
 #pragma unroll
   for (int q = 0; q < kWalkA; ++q) jn[q] = q < w ? a.nbr[s0 + (int64_t)q * kChunk] : -1;
@@ -271,8 +292,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
     int j[kWalkA];
     double uj[kWalkA], vj[kWalkA];
     double2 t[kWalkA];
-    float2 uj32[kWalkA];
-    float r2[kWalkA];
+    float2 uj32[kWalkA], e32[kWalkA];
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
       j[q] = jn[q];
@@ -283,7 +303,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
       if (HG) vj[q] = a.vol[jj];
       if (BREAK) {
         uj32[q] = a.u32[jj];
-        r2[q] = __ldcs(&a.br2[sq]);
+        e32[q] = __ldcs(&a.bxi32[sq]);
       }
     }
 #pragma unroll
@@ -292,15 +312,12 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
       if (j[q] < 0) continue;
-      if (BREAK && !surely_intact(ui32, uj32[q], r2[q])) {
-        const int64_t sq = s + (int64_t)q * kChunk;
-        const double2 e = __ldcs(&a.bxi[sq]), ua = a.u[i], ub = a.u[j[q]];
-        const double dx = ub.x - ua.x, dy = ub.y - ua.y;
-        const double z = fma(dx, fma(2.0, e.x, dx), dy * fma(2.0, e.y, dy));
-        if (z > __ldcs(&a.blim[sq])) {
+      if (BREAK) {
+        const int v = stretch_fp32(ui32, uj32[q], e32[q], s2);
+        if (v <= 0 && (v < 0 || stretch_fp64(a, i, j[q], s + (int64_t)q * kChunk))) {
           // both threads of the pair find the same; the second one does not store, and if it
           // reads the slot after the first one's store it skips the bond there
-          if (h == 0) a.nbr[sq] = -2 - j[q];
+          if (h == 0) a.nbr[s + (int64_t)q * kChunk] = -2 - j[q];
           ++newly;
           continue;
         }

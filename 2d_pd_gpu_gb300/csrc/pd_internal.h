@@ -14,7 +14,7 @@
 //                      a warp is one coalesced 128 B (int) or 512 B (double2)
 //                      line.  nbr int32 (j, -1 padding,
 //                      -2-j broken), bxi double2 (xi = x_j - x_i), bgeo double2
-//                      (V_j xi), blim double (((1+s_c)^2-1) |xi|^2).
+//                      (V_j xi), bxi32 float2 (xi in FP32).
 //   Precomputing the bond geometry trades HBM bytes for FP64 operations: on
 //   GB300 one FP64 operation costs as much time as ~12 bytes of HBM traffic.
 #pragma once
@@ -83,9 +83,8 @@ struct Fp64Args {
   int32_t* nbr;  // the FP64 form's SELL position of particle i is i
   const double2* __restrict__ bxi;
   const double2* __restrict__ bgeo;
-  const double* __restrict__ blim;
-  const float* __restrict__ br2;  // (s_c |xi|)^2 (1 - 1e-5), rounded toward 0: FP32 stretch certificate
-  float2* u32;                    // u rounded to FP32 (shadow for the certificate)
+  const float2* __restrict__ bxi32;  // xi rounded to FP32 (the FP32 stretch test)
+  float2* u32;                       // u rounded to FP32 (shadow for the same)
   double2* hg;  // 2 k_hg sum_j V_j (u_j - u_i), pass A -> pass B
   // pd_step_host: the drift takes the state from page-locked host memory
   // (read over the CPU-GPU link by the kernel itself) and the last pass B
@@ -103,6 +102,7 @@ struct Fp64Args {
   double c11, c12, c33;
   double dt, dt2, inv_rho, det_guard, k_hg, k_hg2, damage_fail;  // k_hg2 = 2 k_hg
   double one, neg_one, neg_zero;  // 1, -1, -0 (add1, sub1, mul1)
+  double s2;                      // stretch limit factor (1 + s_c)^2 - 1 = s_c (2 + s_c)
   unsigned long long* counters;
   int32_t brk;  // bond breaking on (s_c > 0)
   int32_t pad;
@@ -222,10 +222,7 @@ int build_spatial_order(int64_t n, const double2* d_x, const double* h_x, cudaSt
 int build_sell(int64_t n, const int64_t* d_row_ptr, const int32_t* d_col, cudaStream_t s, SellLayout* out,
                unsigned long long* d_counters, std::string* msg);
 void launch_bond_geometry_fp64(int64_t n, const double2* x, const double* vol, const SellLayout& L,
-                               const int64_t* row_ptr, double s_c, double2* bxi, double2* bgeo, double* blim,
-                               float* br2, cudaStream_t s);
-void launch_bond_limit_fp64(int64_t nslots, const double2* bxi, double s_c, const int32_t* nbr, double* blim,
-                            float* br2, cudaStream_t s);
+                               double2* bxi, double2* bgeo, float2* bxi32, cudaStream_t s);
 void launch_mask_out(int64_t n, const int64_t* row_ptr, const int32_t* col, const SellLayout& L, uint8_t* alive,
                      cudaStream_t s);
 void launch_sell_reset(int64_t n, const int64_t* row_ptr, const int32_t* col, const SellLayout& L, cudaStream_t s);
