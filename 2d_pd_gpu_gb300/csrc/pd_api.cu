@@ -62,6 +62,7 @@ struct pd_ctx {
   double2* ba_kq0 = nullptr;  // K_b^-1 with its det-guard flag
   double2* ba_kq1 = nullptr;
   double* ba_wtri = nullptr;  // and, per particle, its weight matrix's lower triangle
+  double* ba_rv = nullptr;    // and 1 / its family's volume
   int32_t max_family = 0;
   // pd_step_host's copy / compute pipeline (streams and events, see plan_slabs)
   cudaStream_t io[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -79,6 +80,8 @@ struct pd_ctx {
   // Mazars damage history (pd_mazars_*)
   double *mz_thr = nullptr, *mz_bd = nullptr, *mz_status = nullptr;
   pd_mazars_params mz{};
+  double2 *mz_tt = nullptr, *mz_kq0 = nullptr, *mz_kq1 = nullptr;  // k_mz_table's (bond-associated weights)
+  bool mz_table_ok = false, mz_table_none = false;  // formed for the current parameters; too large, not kept
   // counters (device) + host mirror of steps
   unsigned long long* counters = nullptr;
   int64_t steps = 0;
@@ -177,6 +180,10 @@ void free_families(pd_ctx* c) {
   dfree(c->mz_thr);
   dfree(c->mz_bd);
   dfree(c->mz_status);
+  dfree(c->mz_tt);
+  dfree(c->mz_kq0);
+  dfree(c->mz_kq1);
+  c->mz_table_ok = c->mz_table_none = false;
   dfree(c->halo.visit);
   dfree(c->halo.loc);
   dfree(c->halo.loc0);
@@ -194,6 +201,7 @@ void free_families(pd_ctx* c) {
   dfree(c->ba_kq0);
   dfree(c->ba_kq1);
   dfree(c->ba_wtri);
+  dfree(c->ba_rv);
   c->sell = pd::SellLayout{};
   c->slab_bnd.clear();
   c->slab_need.clear();
@@ -290,6 +298,7 @@ pd::BondAssoc ba_args(pd_ctx* c) {
   b.kq0 = c->ba_kq0;
   b.kq1 = c->ba_kq1;
   b.wtri = c->ba_wtri;
+  b.rv = c->ba_rv;
   return b;
 }
 
@@ -310,6 +319,7 @@ int ensure_ba(pd_ctx* c) {
   if (!c->ba_ex) PD_CK(c, cudaMalloc(&c->ba_ex, ns * sizeof(double2)));
   if (!c->ba_kq0) PD_CK(c, cudaMalloc(&c->ba_kq0, ns * sizeof(double2)));
   if (!c->ba_kq1) PD_CK(c, cudaMalloc(&c->ba_kq1, ns * sizeof(double2)));
+  if (!c->ba_rv) PD_CK(c, cudaMalloc(&c->ba_rv, (size_t)(c->n > 0 ? c->n : 1) * sizeof(double)));
   if (!c->ba_wtri)
     PD_CK(c, cudaMalloc(&c->ba_wtri, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaTri * sizeof(double)));
   pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
@@ -586,6 +596,7 @@ int pd_set_params(pd_ctx* c, const pd_params* p) {
   PD_CK(c, cudaSetDevice(c->p.device));
   c->p = *p;
   c->c_override = false;
+  c->mz_table_ok = false;
   clear_graphs(c);
   if (c->has_families) {
     int rc2 = upload_gvel(c);
@@ -991,10 +1002,39 @@ pd::MazarsArgs mazars_args(pd_ctx* c) {
   m.thr = c->mz_thr;
   m.bd = c->mz_bd;
   m.status = c->mz_status;
+  if (c->mz_table_ok) {
+    m.tt = c->mz_tt;
+    m.kq0 = c->mz_kq0;
+    m.kq1 = c->mz_kq1;
+  }
   return m;
 }
 
 bool bond_associated(const pd_ctx* c) { return c->p.n1 != 0.0 || c->p.n2 != 0.0; }
+
+// The bond-associated update's weight table (16 KB per particle), formed for the current
+// parameters on first use.  Where it would take more than a quarter of the free memory, the
+// updates evaluate the weights themselves.
+void ensure_mazars_table(pd_ctx* c) {
+  if (!bond_associated(c) || c->mz_table_ok || c->mz_table_none || c->n == 0) return;
+  const size_t bytes = (size_t)c->n * 1024 * sizeof(double2), ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
+  if (!c->mz_kq1) {
+    size_t free_b = 0, total_b = 0;
+    bool ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes / 3 < free_b / 12;
+    ok = ok && cudaMalloc(&c->mz_tt, bytes) == cudaSuccess && cudaMalloc(&c->mz_kq0, ns * sizeof(double2)) == cudaSuccess &&
+         cudaMalloc(&c->mz_kq1, ns * sizeof(double2)) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      dfree(c->mz_tt);
+      dfree(c->mz_kq0);
+      dfree(c->mz_kq1);
+      c->mz_table_none = true;
+      return;
+    }
+  }
+  c->mz_table_ok = true;
+  pd::launch_mazars_table(fp64_args(c), ba_args(c), mazars_args(c), c->stream);
+}
 
 }  // namespace
 
@@ -1034,6 +1074,7 @@ int pd_mazars_update(pd_ctx* c) {
   if (!c->mz_thr) return fail(c, PD_ERR_ORDER, "pd_mazars_init first");
   PD_CK(c, cudaSetDevice(c->p.device));
   const pd::BondAssoc ba = ba_args(c);
+  ensure_mazars_table(c);
   pd::launch_mazars_update(fp64_args(c), bond_associated(c) ? &ba : nullptr, mazars_args(c), c->stream);
   PD_CK(c, cudaGetLastError());
   return PD_OK;

@@ -118,6 +118,7 @@ struct BondAssoc {
   double2* kq0;    // per bond slot: K_b^-1 (q11, q12)
   double2* kq1;    // per bond slot: (q22, 1 if K_b fails the det guard else 0)
   double* wtri;    // per particle with <= 32 bonds: its weight matrix's lower triangle (kBaTri doubles)
+  double* rv;      // per particle: 1 / its family's volume
 };
 constexpr int64_t kBaTri = 32 * 33 / 2;
 
@@ -127,6 +128,10 @@ struct MazarsArgs {
   double* thr;     // per SELL slot: history threshold
   double* bd;      // per SELL slot: bond damage
   double* status;  // per particle: sum of bond damage / family size
+  // bond-associated weights (k_mz_table; null: evaluated in every update)
+  double2* tt;     // per particle, 32 x 32: w(b,k) V_k xi_k of bond b = lane at [k][b] (families of <= 32 bonds)
+  double2* kq0;    // per slot: K_b^-1 (q11, q12) over the whole family
+  double2* kq1;    // per slot: (q22, 1 if K_b fails the det guard else 0)
 };
 
 // Chunk a warp runs in the mixed passes: warp w of visiting block b runs
@@ -255,6 +260,7 @@ void launch_ba_pass_b(const Fp64Args& a, const BondAssoc& b, int mode, cudaStrea
 
 // ---- Mazars damage (pd_mazars.cu), FP64 contexts; ba != nullptr: bond-associated weights
 void launch_mazars_reset(int64_t nslots, int64_t n, const MazarsArgs& m, cudaStream_t s);
+void launch_mazars_table(const Fp64Args& a, const BondAssoc& ba, const MazarsArgs& m, cudaStream_t s);
 void launch_mazars_update(const Fp64Args& a, const BondAssoc* ba, const MazarsArgs& m, cudaStream_t s);
 void launch_mazars_to_csr(const Fp64Args& a, const int64_t* row_ptr, const MazarsArgs& m, double* thr_csr,
                           double* bd_csr, cudaStream_t s);
