@@ -18,8 +18,8 @@
 // and the parameters only, so what does not involve the displacements is
 // formed once, at set-up and on every parameter change, by the set-up form of
 // pass A (k_ba_pass_a<true>, after k_ba_bonds): per slot |xi|, 1/|xi|,
-// exp(+-n1 |xi| / l) and K_b^-1 with its det-guard flag; per particle with
-// <= 32 bonds, the lower triangle of its weight matrix.
+// exp(+-n1 |xi| / l) and K_b^-1 with its det-guard flag; per particle, 1 / V_h
+// and, with <= 32 bonds, the lower triangle of its weight matrix.
 //
 // Pass A runs one warp per particle and one lane per bond (families <= 64
 // bonds, two per lane): the family's bond data is staged in shared memory,
@@ -235,12 +235,16 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
     F.P[q][2] = vq * fma(s12, q11, s22 * q12);
     F.P[q][3] = vq * fma(s12, q12, s22 * q22);
   }
-  if (KTAB) return;
-  // V_h in family order (as the oracle), then T_ij of bond jj
-  double vh = 0.0;
-  for (int k = 0; k < n; ++k) vh = vh + F.vv[k];
+  if (KTAB) {
+    if (lane == 0) {  // V_h in family order (as the oracle)
+      double vh = 0.0;
+      for (int k = 0; k < n; ++k) vh = vh + F.vv[k];
+      b.rv[i] = 1.0 / vh;
+    }
+    return;
+  }
   __syncwarp();
-  const double rv = 1.0 / vh;
+  const double rv = b.rv[i];
   for (int jj = lane; jj < n; jj += 32) {
     double m11 = 0.0, m12 = 0.0, m21 = 0.0, m22 = 0.0;
     for (int q = 0; q < n; ++q) {
@@ -256,60 +260,70 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
   }
 }
 
-// Velocity BC, drift, fixed BC (as pd_fp64.cu's drift_one).
-__device__ __forceinline__ void ba_drift(const Fp64Args& a, int64_t i, double2& v, double2& u, double anx,
-                                         double any) {
-  const int g = a.bc[i];
-  const int kind = g ? a.gkind[g - 1] : PD_BC_NONE;
-  if (kind == PD_BC_VELOCITY) v = a.gval[g - 1];
-  u.x = u.x + (v.x * a.dt + (0.5 * anx) * a.dt2);
-  u.y = u.y + (v.y * a.dt + (0.5 * any) * a.dt2);
-  if (kind == PD_BC_FIXED) u = make_double2(0.0, 0.0);
-}
+// Pass B, two threads per particle (component h each) and kBaWalk bonds at a
+// time, whose loads are in flight together: with one thread per particle and
+// one bond at a time the reference's mesh kept 17 blocks waiting on ~56
+// dependent loads in turn (37 us; its data takes ~2 us to read).
+constexpr int kBaWalk = 4;
+constexpr int kBaPairBlock = 64;
 
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) k_ba_pass_b(Fp64Args a, BondAssoc b) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kBaPairBlock) k_ba_pass_b(Fp64Args a, BondAssoc b) {
+  const int64_t i = (int64_t)blockIdx.x * (kBaPairBlock / 2) + (threadIdx.x >> 1);
+  const int h = threadIdx.x & 1;
   if (i >= a.n) return;
   const int64_t c0 = i >> 5;
   const int w = a.chunk_w[c0];
   const int64_t s0 = a.chunk_base[c0] + (i & 31);
-  double fx = 0.0, fy = 0.0;
-  for (int k = 0; k < w; ++k) {
-    const int64_t s = s0 + (int64_t)k * kChunk;
-    const int j = a.nbr[s];
-    if (j < 0) continue;
-    const double2 tij = b.tb[s], tji = b.tb[b.rslot[s]];
-    const double vj = a.vol[j];
-    fx = fma(tij.x - tji.x, vj, fx);
-    fy = fma(tij.y - tji.y, vj, fy);
+  auto comp = [h](const double2* p, int64_t k) { return reinterpret_cast<const double*>(p)[2 * k + h]; };
+  auto put = [h](double2* p, int64_t k, double x) { reinterpret_cast<double*>(p)[2 * k + h] = x; };
+  double v = comp(a.v, i), ao = comp(MODE == 2 ? a.acc : a.f, i), u = comp(a.u, i);
+  double f = 0.0;
+  int jn[kBaWalk];
+  int64_t rn[kBaWalk];
+  auto ask = [&](int k0) {  // neighbours and reverse slots of slots k0 .. (-1: none)
+#pragma unroll
+    for (int q = 0; q < kBaWalk; ++q) {
+      const int64_t s = s0 + (int64_t)(k0 + q) * kChunk;
+      jn[q] = k0 + q < w ? a.nbr[s] : -1;
+      rn[q] = k0 + q < w ? b.rslot[s] : s0;
+    }
+  };
+  ask(0);
+  for (int k = 0; k < w; k += kBaWalk) {
+    int j[kBaWalk];
+    double tij[kBaWalk], tji[kBaWalk], vj[kBaWalk];
+#pragma unroll
+    for (int q = 0; q < kBaWalk; ++q) {
+      j[q] = jn[q];
+      const bool on = j[q] >= 0;
+      tij[q] = comp(b.tb, on ? s0 + (int64_t)(k + q) * kChunk : s0);
+      tji[q] = comp(b.tb, on ? rn[q] : s0);
+      vj[q] = a.vol[on ? (int64_t)j[q] : i];
+    }
+    ask(k + kBaWalk);
+#pragma unroll
+    for (int q = 0; q < kBaWalk; ++q)
+      if (j[q] >= 0) f = fma(tij[q] - tji[q], vj[q], f);
   }
-  double2 v = a.v[i];
-  double aox, aoy;
-  if (MODE == 2) {
-    const double2 ao = a.acc[i];
-    aox = ao.x;
-    aoy = ao.y;
-  } else {
-    const double2 fo = a.f[i];
-    aox = fo.x * a.inv_rho;
-    aoy = fo.y * a.inv_rho;
+  if (MODE != 2) ao = ao * a.inv_rho;
+  const double an = f * a.inv_rho;
+  v = v + (0.5 * (ao + an)) * a.dt;
+  put(a.f, i, f);
+  if (MODE == 2) put(a.acc, i, an);
+  if (MODE == 1) {  // velocity BC, drift, fixed BC (as pd_fp64.cu's drift_one)
+    const int g = a.bc[i];
+    const int kind = g ? a.gkind[g - 1] : PD_BC_NONE;
+    if (kind == PD_BC_VELOCITY) v = comp(a.gval, g - 1);
+    u = u + (v * a.dt + (0.5 * an) * a.dt2);
+    if (kind == PD_BC_FIXED) u = 0.0;
+    put(a.u, i, u);
   }
-  const double anx = fx * a.inv_rho, any = fy * a.inv_rho;
-  v.x = v.x + (0.5 * (aox + anx)) * a.dt;
-  v.y = v.y + (0.5 * (aoy + any)) * a.dt;
-  a.f[i] = make_double2(fx, fy);
-  if (MODE == 2) a.acc[i] = make_double2(anx, any);
-  if (MODE == 1) {
-    double2 u = a.u[i];
-    ba_drift(a, i, v, u, anx, any);
-    a.u[i] = u;
-  }
-  a.v[i] = v;
+  put(a.v, i, v);
   if (a.out_v) {  // pd_step_host's last pass
-    a.out_u[i] = a.u[i];
-    a.out_v[i] = v;
-    a.out_f[i] = make_double2(fx, fy);
+    put(a.out_u, i, u);
+    put(a.out_v, i, v);
+    put(a.out_f, i, f);
   }
 }
 
@@ -370,13 +384,13 @@ void launch_ba_pass_a(const Fp64Args& a, const BondAssoc& b, cudaStream_t s) {
 
 void launch_ba_pass_b(const Fp64Args& a, const BondAssoc& b, int mode, cudaStream_t s) {
   if (a.n <= 0) return;
-  const unsigned nb = (unsigned)blocks_for(a.n);
+  const unsigned nb = (unsigned)blocks_for(2 * a.n, kBaPairBlock);
   if (mode == 0)
-    k_ba_pass_b<0><<<nb, kBlock, 0, s>>>(a, b);
+    k_ba_pass_b<0><<<nb, kBaPairBlock, 0, s>>>(a, b);
   else if (mode == 1)
-    k_ba_pass_b<1><<<nb, kBlock, 0, s>>>(a, b);
+    k_ba_pass_b<1><<<nb, kBaPairBlock, 0, s>>>(a, b);
   else
-    k_ba_pass_b<2><<<nb, kBlock, 0, s>>>(a, b);
+    k_ba_pass_b<2><<<nb, kBaPairBlock, 0, s>>>(a, b);
 }
 
 }  // namespace pd
