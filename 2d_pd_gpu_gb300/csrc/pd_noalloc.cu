@@ -33,7 +33,8 @@
 
 namespace {
 
-constexpr int kNoallocBlock = 256;
+constexpr int kNoallocBlock = 64;  // 32 particles: small blocks spread a small call over the chip
+
 constexpr int kScratchPerParticle = 8;  // W (4) + m / V (2) + penalty term (2)
 
 // The scratch.  Every call shares it and it keeps the previous call's
@@ -57,6 +58,7 @@ struct NoallocArgs {
   double2* mt;   // scratch
   double2* hg;   // scratch
   double c11, c12, c33, dt, inv_rho, det_guard, k_hg;
+  double one, neg_one, neg_zero;  // 1, -1, -0
 };
 
 // A particle's row [r0, r1) is walkable when it lies inside [0, row_ptr[n]]
@@ -67,101 +69,234 @@ __device__ __forceinline__ bool row_ok(const NoallocArgs& a, int64_t i, int64_t*
   return a.row_ptr[0] == 0 && 0 <= *r0 && *r0 <= *r1 && *r1 <= a.row_ptr[a.n];
 }
 
+// A value in a register: a DFMA of three registers takes 16 cycles of the FP64
+// pipe per warp and SM, a DADD, DMUL or DFMA with a constant operand 19, so the
+// bond loops write x - y = fma(y, -1, x), x + y = fma(x, 1, y), x y = fma(x, y, -0)
+// (one rounding of the same value each): a call on 256 x 255 particles 104 -> 91 us.
+__device__ __forceinline__ double in_register(double x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+// The warp's longest row (the pair exchanges of a walk run in every lane).
+__device__ __forceinline__ int64_t longest(int64_t len) {
+  for (int o = 16; o; o >>= 1) {
+    const int64_t t = __shfl_xor_sync(0xffffffffu, len, o);
+    len = t > len ? t : len;
+  }
+  return len;
+}
+
+// Stress and W of particle i from its sums: row h of D (d1, d2), K^-1; the
+// lanes of a particle's pair exchange what the symmetric stress needs.  All
+// lanes of the warp call it.
+__device__ __forceinline__ double2 w_row(const NoallocArgs& a, int h, double d1, double d2, double q11, double q12,
+                                         double q22, double vi) {
+  const double g1 = fma(d1, q11, d2 * q12), g2 = fma(d1, q12, d2 * q22);
+  const double diag = h ? g2 : g1, other = __shfl_xor_sync(0xffffffffu, diag, 1);
+  const double off = h ? g1 : g2, cross = __shfl_xor_sync(0xffffffffu, off, 1);
+  const double e11 = h ? other : diag, e22 = h ? diag : other, e12 = 0.5 * (off + cross);
+  const double sd = fma(h ? a.c12 : a.c11, e11, (h ? a.c11 : a.c12) * e22);
+  const double s12 = a.c33 * e12;
+  const double sa = h ? s12 : sd, sb = h ? sd : s12, kh = -a.k_hg;
+  return make_double2(vi * fma(kh, g1, fma(sa, q11, sb * q12)), vi * fma(kh, g2, fma(sa, q12, sb * q22)));
+}
+
+// What pass A leaves of component h of particle i.  singular: no stress.
+__device__ __forceinline__ void store_a(const NoallocArgs& a, int64_t i, int h, bool ok, bool singular, double hg,
+                                        double mt, double2 W) {
+  const double q = nan("");
+  if (!ok) hg = mt = W.x = W.y = q;
+  else if (singular) mt = W.x = W.y = 0.0;
+  reinterpret_cast<double*>(a.hg)[2 * i + h] = hg;
+  reinterpret_cast<double*>(a.mt)[2 * i + h] = mt;
+  (h ? a.w23 : a.w01)[i] = W;
+}
+
 // Pass A: K^-1 and m/V over the given family, D, stress, W (no bond breaking).
+// Two threads per particle, thread h summing component h (k11, k12 or k22; m_h,
+// row h of D, the penalty's h): 9 of the 17 FP64 operations of a bond each, the
+// sums in family order as ever.  An FP64 instruction keeps its SM quarter busy
+// for 64 cycles, so a thread's chain is what a call waits for.
+constexpr int kNoallocWalk = 4;  // bonds in flight per thread (2: 24.0 us against 21.6 per 30 x 31 call)
+
 __global__ void __launch_bounds__(kNoallocBlock) k_noalloc_pass_a(NoallocArgs a) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+  const int64_t p = (int64_t)blockIdx.x * (kNoallocBlock / 2) + (threadIdx.x >> 1);
+  const int h = threadIdx.x & 1;
+  const bool have = p < a.n;
+  const int64_t i = have ? p : a.n - 1;  // (a lane past the end repeats the last particle and stores nothing)
+  const double xi = reinterpret_cast<const double*>(a.x)[2 * i + h], ui = reinterpret_cast<const double*>(a.u)[2 * i + h];
+  int64_t r0, r1;
+  bool ok = row_ok(a, i, &r0, &r1);
+  double ka = 0.0, kb = 0.0, m = 0.0;     // h = 0: k11, k12; h = 1: k22 (in kb)
+  double d1 = 0.0, d2 = 0.0, ah = 0.0;
+  const int64_t len = ok ? r1 - r0 : 0;
+  const double one = in_register(a.one), neg1 = in_register(a.neg_one), neg0 = in_register(a.neg_zero);
+  const int64_t most = longest(len);
+  int jn[kNoallocWalk];
+  auto ask = [&](int64_t k0) {
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) jn[q] = k0 + q < len ? a.col[r0 + k0 + q] : (int)i;
+  };
+  ask(0);
+  for (int64_t k = 0; k < most; k += kNoallocWalk) {
+    double xj[kNoallocWalk], uj[kNoallocWalk], vj[kNoallocWalk];
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) {
+      int j = jn[q];
+      if (j < 0 || j >= a.n) {  // a bad index: read nothing of it, poison this particle
+        ok = false;
+        j = (int)i;
+      }
+      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j + h];
+      uj[q] = reinterpret_cast<const double*>(a.u)[2 * (int64_t)j + h];
+      vj[q] = a.vol[j];
+    }
+    ask(k + kNoallocWalk);
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) {
+      const double e = fma(xi, neg1, xj[q]), t = fma(vj[q], e, neg0);
+      const double e2 = __shfl_xor_sync(0xffffffffu, e, 1), t2 = __shfl_xor_sync(0xffffffffu, t, 1);
+      if (k + q < len) {
+        const double tx = h ? t2 : t, ty = h ? t : t2;
+        ka = fma(t, e, ka);           // k11 | k22
+        if (h == 0) kb = fma(t, e2, kb);  // k12
+        m = fma(t, one, m);
+        const double d = fma(ui, neg1, uj[q]);
+        d1 = fma(d, tx, d1);
+        d2 = fma(d, ty, d2);
+        ah = fma(vj[q], d, ah);
+      }
+    }
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const double k11 = __shfl_sync(0xffffffffu, ka, threadIdx.x & 30), k12 = __shfl_sync(0xffffffffu, kb, threadIdx.x & 30),
+               k22 = __shfl_sync(0xffffffffu, ka, (threadIdx.x & 30) + 1);
+  const double det = fma(k11, k22, -(k12 * k12));
+  const bool singular = r1 == r0 || !(det > a.det_guard * (k11 * k22));
+  const double vi = a.vol[i], quo = 1.0 / (h ? vi : det);
+  const double r = __shfl_sync(0xffffffffu, quo, threadIdx.x & 30), rv = __shfl_sync(0xffffffffu, quo, (threadIdx.x & 30) + 1);
+  const double2 W = w_row(a, h, d1, d2, k22 * r, -k12 * r, k11 * r, vi);
+  if (have) store_a(a, i, h, ok, singular, (2.0 * a.k_hg) * ah, m * rv, W);
+}
+
+// Pass A of a small call: 16 lanes per particle.  The lanes take 16 bonds at a
+// time, form each bond's xi, V xi, d (6 operations, one bond per lane) into
+// shared memory, and then 11 of them run one of the 11 sums each over these
+// bonds, in family order: a chain of ~40 FP64 operations per particle instead
+// of ~290.  It costs twice the two-thread form's FP64 issue per particle, so it
+// serves the calls that leave most of the chip idle.
+constexpr int kNoallocSmallBlock = 64;
+constexpr int kNoallocSmall = 4096;
+
+__global__ void __launch_bounds__(kNoallocSmallBlock) k_noalloc_pass_a_small(NoallocArgs a) {
+  enum { EX, EY, T0, T1, DX, DY, V, NV };
+  __shared__ double val[kNoallocSmallBlock / 16][NV][16];
+  const int64_t p = (int64_t)blockIdx.x * (kNoallocSmallBlock / 16) + (threadIdx.x >> 4);
+  const int c = threadIdx.x & 15;
+  const bool have = p < a.n;
+  const int64_t i = have ? p : a.n - 1;
+  double(*S)[16] = val[threadIdx.x >> 4];
+  // sum c adds S[pc] * S[qc] (sums 3 and 4, of m: S[pc] * 1, which is S[pc])
+  const int pc = c < 2 ? T0 : c == 2 ? T1 : c == 3 ? T0 : c == 4 ? T1 : c < 7 ? DX : c < 9 ? DY : V;
+  const int qc = c == 0 ? EX : c < 3 ? EY : c == 5 || c == 7 ? T0 : c < 9 ? T1 : c == 9 ? DX : DY;
+  const bool sums_m = c == 3 || c == 4;
   const double2 xi = a.x[i], ui = a.u[i];
   int64_t r0, r1;
   bool ok = row_ok(a, i, &r0, &r1);
-  double k11 = 0.0, k12 = 0.0, k22 = 0.0, mx = 0.0, my = 0.0;
-  double d11 = 0.0, d12 = 0.0, d21 = 0.0, d22 = 0.0, ax = 0.0, ay = 0.0;
-  for (int64_t s = r0; ok && s < r1; ++s) {
-    const int j = a.col[s];
-    if (j < 0 || j >= a.n) {  // a bad index: read nothing, poison this particle
-      ok = false;
-      break;
+  const int64_t len = ok ? r1 - r0 : 0;
+  int64_t most = len;  // of the warp's two particles
+  const int64_t t = __shfl_xor_sync(0xffffffffu, most, 16);
+  most = t > most ? t : most;
+  double sum = 0.0;
+  for (int64_t k0 = 0; k0 < most; k0 += 16) {
+    if (k0 + c < len) {
+      int j = a.col[r0 + k0 + c];
+      if (j < 0 || j >= a.n) {
+        ok = false;
+        j = (int)i;
+      }
+      const double2 xj = a.x[j], uj = a.u[j];
+      const double vj = a.vol[j], ex = xj.x - xi.x, ey = xj.y - xi.y;
+      S[EX][c] = ex;
+      S[EY][c] = ey;
+      S[T0][c] = vj * ex;
+      S[T1][c] = vj * ey;
+      S[DX][c] = uj.x - ui.x;
+      S[DY][c] = uj.y - ui.y;
+      S[V][c] = vj;
     }
-    const double2 xj = a.x[j], uj = a.u[j];
-    const double ex = xj.x - xi.x, ey = xj.y - xi.y;
-    const double vj = a.vol[j];
-    const double t0 = vj * ex, t1 = vj * ey;
-    k11 = fma(t0, ex, k11);
-    k12 = fma(t0, ey, k12);
-    k22 = fma(t1, ey, k22);
-    mx = mx + t0;
-    my = my + t1;
-    const double dx = uj.x - ui.x, dy = uj.y - ui.y;
-    d11 = fma(dx, t0, d11);
-    d12 = fma(dx, t1, d12);
-    d21 = fma(dy, t0, d21);
-    d22 = fma(dy, t1, d22);
-    ax = fma(vj, dx, ax);
-    ay = fma(vj, dy, ay);
+    __syncwarp();
+    const int m = (int)(len - k0 < 16 ? len - k0 : 16);
+    for (int k = 0; k < m; ++k) sum = fma(S[pc][k], sums_m ? 1.0 : S[qc][k], sum);
+    __syncwarp();
   }
-  if (!ok) {
-    const double q = nan("");
-    a.hg[i] = make_double2(q, q);
-    a.w01[i] = make_double2(q, q);
-    a.w23[i] = make_double2(q, q);
-    a.mt[i] = make_double2(q, q);
-    return;
-  }
-  const double k2 = 2.0 * a.k_hg;
-  a.hg[i] = make_double2(k2 * ax, k2 * ay);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int g0 = threadIdx.x & 16, h = c & 1;
+  ok = ((__ballot_sync(0xffffffffu, ok) >> g0) & 0xffffu) == 0xffffu;
+  auto get = [&](int q) { return __shfl_sync(0xffffffffu, sum, g0 + q); };
+  const double k11 = get(0), k12 = get(1), k22 = get(2), m = get(3 + h), d1 = get(5 + 2 * h), d2 = get(6 + 2 * h),
+               ah = get(9 + h);
   const double det = fma(k11, k22, -(k12 * k12));
-  if (r1 == r0 || !(det > a.det_guard * (k11 * k22))) {
-    a.w01[i] = make_double2(0.0, 0.0);
-    a.w23[i] = make_double2(0.0, 0.0);
-    a.mt[i] = make_double2(0.0, 0.0);
-    return;
-  }
-  const double r = 1.0 / det;
-  const double q11 = k22 * r, q12 = -k12 * r, q22 = k11 * r;
-  const double rv = 1.0 / a.vol[i];
-  a.mt[i] = make_double2(mx * rv, my * rv);
-  const double g11 = fma(d11, q11, d12 * q12), g12 = fma(d11, q12, d12 * q22);
-  const double g21 = fma(d21, q11, d22 * q12), g22 = fma(d21, q12, d22 * q22);
-  const double e11 = g11, e22 = g22, e12 = 0.5 * (g12 + g21);
-  const double s11 = fma(a.c11, e11, a.c12 * e22);
-  const double s22 = fma(a.c12, e11, a.c11 * e22);
-  const double s12 = a.c33 * e12;
-  const double vi = a.vol[i], kh = -a.k_hg;
-  a.w01[i] = make_double2(vi * fma(kh, g11, fma(s11, q11, s12 * q12)), vi * fma(kh, g12, fma(s11, q12, s12 * q22)));
-  a.w23[i] = make_double2(vi * fma(kh, g21, fma(s12, q11, s22 * q12)), vi * fma(kh, g22, fma(s12, q12, s22 * q22)));
+  const bool singular = r1 == r0 || !(det > a.det_guard * (k11 * k22));
+  const double vi = a.vol[i], quo = 1.0 / (h ? vi : det);
+  const double r = __shfl_sync(0xffffffffu, quo, g0), rv = __shfl_sync(0xffffffffu, quo, g0 + 1);
+  const double2 W = w_row(a, h, d1, d2, k22 * r, -k12 * r, k11 * r, vi);
+  if (have && c < 2) store_a(a, i, h, ok, singular, (2.0 * a.k_hg) * ah, m * rv, W);
 }
 
-// Pass B: gather force, velocity-Verlet kick, acce := f / rho.
+// Pass B: gather force, velocity-Verlet kick, acce := f / rho; component h of
+// a particle per thread, as pass A.
 __global__ void __launch_bounds__(kNoallocBlock) k_noalloc_pass_b(NoallocArgs a) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const double2 xi = a.x[i], wa = a.w01[i], wb = a.w23[i], m = a.mt[i], h = a.hg[i];
-  double fx = fma(wa.x, m.x, fma(wa.y, m.y, h.x));
-  double fy = fma(wb.x, m.x, fma(wb.y, m.y, h.y));
+  const int64_t p = (int64_t)blockIdx.x * (kNoallocBlock / 2) + (threadIdx.x >> 1);
+  const int h = threadIdx.x & 1;
+  const bool have = p < a.n;
+  const int64_t i = have ? p : a.n - 1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // pass A's scratch
+  const double2* Wr = h ? a.w23 : a.w01;
+  const double2 wi = Wr[i], m = a.mt[i];
+  const double xi = reinterpret_cast<const double*>(a.x)[2 * i + h];
+  const double hg = reinterpret_cast<const double*>(a.hg)[2 * i + h];
+  const double ao = reinterpret_cast<const double*>(a.acc)[2 * i + h];
+  double v = reinterpret_cast<const double*>(a.v)[2 * i + h];
+  double f = fma(wi.x, m.x, fma(wi.y, m.y, hg));
   int64_t r0, r1;
   bool ok = row_ok(a, i, &r0, &r1);
-  for (int64_t s = r0; ok && s < r1; ++s) {
-    const int j = a.col[s];
-    if (j < 0 || j >= a.n) {
-      ok = false;
-      break;
+  const int64_t len = ok ? r1 - r0 : 0, most = longest(len);
+  const double neg1 = in_register(a.neg_one);
+  int jn[kNoallocWalk];
+  auto ask = [&](int64_t k0) {
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) jn[q] = k0 + q < len ? a.col[r0 + k0 + q] : (int)i;
+  };
+  ask(0);
+  for (int64_t k = 0; k < most; k += kNoallocWalk) {
+    double xj[kNoallocWalk];
+    double2 wj[kNoallocWalk];
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) {
+      int j = jn[q];
+      if (j < 0 || j >= a.n) {
+        ok = false;
+        j = (int)i;
+      }
+      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j + h];
+      wj[q] = Wr[j];
     }
-    const double2 xj = a.x[j], ja = a.w01[j], jb = a.w23[j];
-    const double ex = xj.x - xi.x, ey = xj.y - xi.y;
-    fx = fma(ja.x, ex, fx);
-    fx = fma(ja.y, ey, fx);
-    fy = fma(jb.x, ex, fy);
-    fy = fma(jb.y, ey, fy);
+    ask(k + kNoallocWalk);
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) {
+      const double e = fma(xi, neg1, xj[q]), e2 = __shfl_xor_sync(0xffffffffu, e, 1);
+      if (k + q < len) {
+        f = fma(wj[q].x, h ? e2 : e, f);
+        f = fma(wj[q].y, h ? e : e2, f);
+      }
+    }
   }
-  if (!ok) fx = fy = nan("");
-  const double2 ao = a.acc[i];
-  const double anx = fx * a.inv_rho, any = fy * a.inv_rho;
-  double2 v = a.v[i];
-  v.x = v.x + (0.5 * (ao.x + anx)) * a.dt;
-  v.y = v.y + (0.5 * (ao.y + any)) * a.dt;
-  a.v[i] = v;
-  a.f[i] = make_double2(fx, fy);
-  a.acc[i] = make_double2(anx, any);
+  if (!ok) f = nan("");
+  const double an = f * a.inv_rho;
+  v = v + (0.5 * (ao + an)) * a.dt;
+  if (!have) return;
+  reinterpret_cast<double*>(a.v)[2 * i + h] = v;
+  reinterpret_cast<double*>(a.f)[2 * i + h] = f;
+  reinterpret_cast<double*>(a.acc)[2 * i + h] = an;
 }
 
 // Device address of the scratch.  In host code the array's name is only a
@@ -311,11 +446,29 @@ extern "C" int pd_compute_velocity_noalloc(int64_t n, const double* x, const dou
   a.inv_rho = 1.0 / p->rho;
   a.det_guard = p->det_guard;
   a.k_hg = p->k_hg;
+  a.one = 1.0;
+  a.neg_one = -1.0;
+  a.neg_zero = -0.0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned nb = (unsigned)((n + kNoallocBlock - 1) / kNoallocBlock);
-  k_noalloc_pass_a<<<nb, kNoallocBlock, 0, s>>>(a);
-  k_noalloc_pass_b<<<nb, kNoallocBlock, 0, s>>>(a);
+  if (n <= kNoallocSmall) {
+    constexpr int per = kNoallocSmallBlock / 16;
+    k_noalloc_pass_a_small<<<(unsigned)((n + per - 1) / per), kNoallocSmallBlock, 0, s>>>(a);
+  } else {
+    k_noalloc_pass_a<<<(unsigned)((2 * n + kNoallocBlock - 1) / kNoallocBlock), kNoallocBlock, 0, s>>>(a);
+  }
   e = cudaGetLastError();
+  if (e == cudaSuccess) {  // pass B's blocks start while pass A drains, and wait for it
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)((2 * n + kNoallocBlock - 1) / kNoallocBlock));
+    lc.blockDim = dim3(kNoallocBlock);
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    e = cudaLaunchKernelEx(&lc, k_noalloc_pass_b, a);
+  }
   if (e != cudaSuccess) {
     char m[200];
     std::snprintf(m, sizeof(m), "pd_compute_velocity_noalloc: launch: %s", cudaGetErrorString(e));
