@@ -388,7 +388,7 @@ pd::MixedArgs mixed_args(pd_ctx* c) {
   a.damage_fail = c->p.damage_fail;
   a.counters = c->counters;
   a.brk = c->p.s_c > 0.0;
-  a.wmax = c->max_family;
+  a.wmax = std::max(c->max_family, 8);  // (a warp's index chunk is at least 512 B: pass_a_core's spare)
   return a;
 }
 

@@ -16,6 +16,7 @@
 // products.  Nothing here is bit-identical to the FP64 form; its error is
 // measured against it (tests/test_gpu_mixed.py, bench.py).
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "pd_internal.h"
@@ -109,6 +110,111 @@ __device__ void kinv_update_mixed(const MixedArgs& a, int64_t i, int64_t p, int6
   a.singular[p] = 0;
 }
 
+// W^ = V^ (sigma^ K^-1 - k^ G) of a particle from its D (D1 = (d11, d12), D2 =
+// (d21, d22)) and geo, stored by columns {W11, W21, W12, W22}.
+__device__ __forceinline__ float4 w_of(const MixedArgs& a, float2 D1, float2 D2, float4 g) {
+  const float d11 = D1.x, d12 = D1.y, d21 = D2.x, d22 = D2.y;
+  const float k11 = g.x, k12 = g.y, k22 = g.z, vi = g.w;
+  const float g11 = fmaf(d11, k11, d12 * k12), g12 = fmaf(d11, k12, d12 * k22);
+  const float g21 = fmaf(d21, k11, d22 * k12), g22 = fmaf(d21, k12, d22 * k22);
+  const float e11 = g11, e22 = g22, e12 = 0.5f * (g12 + g21);
+  const float s11 = fmaf(a.c11, e11, a.c12 * e22);
+  const float s22 = fmaf(a.c12, e11, a.c11 * e22);
+  const float s12 = a.c33 * e12;
+  const float kh = -a.k_hg;
+  return make_float4(vi * fmaf(kh, g11, fmaf(s11, k11, s12 * k12)), vi * fmaf(kh, g21, fmaf(s12, k11, s22 * k12)),
+                     vi * fmaf(kh, g12, fmaf(s11, k12, s12 * k22)), vi * fmaf(kh, g22, fmaf(s12, k12, s22 * k22)));
+}
+
+// Pass A's update of the particles that lost bonds (newly > 0 in their lane, p
+// its SELL position, s0 and w its slots): broken count, damage, K^-1, m^ and W^, by the whole warp;
+// D: the lanes' sums in shared memory (the call has few registers to save then).
+// Eight lanes take a particle, four particles at a time: each lane requests
+// four of its first 32 bonds at once and forms their terms, lanes 0 .. 4 each
+// sum one of k11, k12, k22, mx, my over all of them in slot order, and lanes
+// 0 .. 3 share one division: kinv_update_mixed's operations.  One thread alone
+// waits for ~56 dependent loads and ~300 FP64 operations (64 cycles each), and
+// its pass waits for it.
+__device__ __noinline__ void kinv_update_mixed_warp(const MixedArgs& a, int64_t p, int64_t s0, int w, int newly,
+                                                    const float4* D) {
+  constexpr int kPer = 4;  // bonds per lane and round
+  const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
+  unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
+  while (todo) {
+    unsigned rest = todo;  // this lane's particle: that of the (lane / 8)-th lane left to do
+    for (int q = lane >> 3; q > 0; --q) rest &= rest - 1;
+    const bool have = rest != 0;
+    const int src = have ? __ffs((int)rest) - 1 : 0;
+    const int64_t gp = __shfl_sync(0xffffffffu, p, src);
+    const int gn = __shfl_sync(0xffffffffu, newly, src);
+    const int64_t i = have ? (int64_t)a.member[gp] : 0;
+    const int64_t gs = __shfl_sync(0xffffffffu, s0, src);
+    const int sw = __shfl_sync(0xffffffffu, w, src), gw = have ? sw : 0;
+    const double2 xi = a.x[i];
+    const double voli = a.vol[i];
+    const int32_t broken = a.broken[i] + gn, fam = a.fam[i];
+    double sum = 0.0;
+    int nal = 0;
+    const int most = __reduce_max_sync(0xffffffffu, gw);
+    for (int k0 = 0; k0 < most; k0 += 8 * kPer) {
+      int j[kPer];
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        const int k = k0 + 8 * r + c;
+        j[r] = k < gw ? a.nbr[gs + (int64_t)k * kChunk] : -1;
+      }
+      double2 xj[kPer];
+      double vj[kPer];
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        xj[r] = a.x[j[r] < 0 ? i : (int64_t)j[r]];
+        vj[r] = a.vol[j[r] < 0 ? i : (int64_t)j[r]];
+      }
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        if (k0 + 8 * r >= most) break;
+        const double ex = (xj[r].x - xi.x) * a.inv_ls, ey = (xj[r].y - xi.y) * a.inv_ls;
+        const double v = vj[r] * a.inv_vs, t0 = v * ex, t1 = v * ey;
+        const unsigned live = __ballot_sync(0xffffffffu, j[r] >= 0) >> g0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const double b0 = __shfl_sync(0xffffffffu, t0, g0 + q), b1 = __shfl_sync(0xffffffffu, t1, g0 + q);
+          const double bx = __shfl_sync(0xffffffffu, ex, g0 + q), by = __shfl_sync(0xffffffffu, ey, g0 + q);
+          const double P = c == 2 || c == 4 ? b1 : b0, Q = c == 0 ? bx : c < 3 ? by : 1.0;
+          if (live >> q & 1) {
+            sum = fma(P, Q, sum);
+            ++nal;
+          }
+        }
+      }
+    }
+    const double k11 = __shfl_sync(0xffffffffu, sum, g0), k12 = __shfl_sync(0xffffffffu, sum, g0 + 1),
+                 k22 = __shfl_sync(0xffffffffu, sum, g0 + 2), mx = __shfl_sync(0xffffffffu, sum, g0 + 3),
+                 my = __shfl_sync(0xffffffffu, sum, g0 + 4);
+    const double det = fma(k11, k22, -(k12 * k12));
+    const double vi = voli * a.inv_vs;
+    const double quo = (c == 0 ? 1.0 : c == 1 ? mx : c == 2 ? my : (double)broken) /
+                       (c == 0 ? det : c < 3 ? vi : (double)fam);
+    const double r = __shfl_sync(0xffffffffu, quo, g0), m0 = __shfl_sync(0xffffffffu, quo, g0 + 1),
+                 m1 = __shfl_sync(0xffffffffu, quo, g0 + 2), damage = __shfl_sync(0xffffffffu, quo, g0 + 3);
+    if (have && c == 0) {
+      const bool bad = nal == 0 || damage > a.damage_fail || !(det > a.det_guard * (k11 * k22));
+      a.broken[i] = broken;
+      a.damage[i] = damage;
+      const float4 geo = bad ? make_float4(0.f, 0.f, 0.f, (float)vi)
+                             : make_float4((float)(k22 * r), (float)(-k12 * r), (float)(k11 * r), (float)vi);
+      a.geo[gp] = geo;
+      a.mh[gp] = bad ? make_float2(0.f, 0.f) : make_float2((float)m0, (float)m1);
+      a.singular[gp] = bad ? 1 : 0;
+      const float4 d = D[src];
+      a.ws[gp] = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, f2(d.x, d.y), f2(d.z, d.w), geo);
+      atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)gn);
+      if (bad) atomicAdd(a.counters + CNT_SINGULAR, 1ull);
+    }
+    for (int q = 0; q < 4 && todo; ++q) todo &= todo - 1;
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) k_init_geometry_mixed(MixedArgs a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -169,6 +275,10 @@ __global__ void __launch_bounds__(kBlock) k_drift_mixed(MixedArgs a) {
   if (p < a.npos) drift_particle_mixed(a, p);
 }
 
+// Slots per group of the walks (1M-particle plate, breaking: pass A 2, 3, 4
+// 51.5, 51.6, 50.9 us; 4M: 166, 163, 159; pass B 2, 4, 7: 49.9, 47.5, 53.5).
+constexpr int kWalkA = 4, kWalkB = 4;
+
 // Neighbour data gathered by the two passes.
 struct NbA {
   float4 u, x;
@@ -196,70 +306,82 @@ __device__ __forceinline__ PreA load_a(const MixedArgs& a, int64_t p) {
 // UV: every particle's V^ is 1 (uniform volumes; the host checks that
 // (float)(V_i / Vs) == 1 for all i): the V^ gathers and products are left
 // out, which changes no result -- x * 1 and fma(1, x, y) are exact.
+// live: the lane has a particle (the whole warp calls it); spare: 512 B of the
+// warp's shared memory for the end of the walk.
 template <bool BREAK, bool UV, typename Idx, typename Gather>
-__device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, const PreA& pre, int w, int64_t s0, Idx idx,
-                                            Gather gather) {
+__device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, bool live, const PreA& pre, int w, int64_t s0,
+                                            Idx idx, Gather gather, float4* spare) {
   const float4 ui = pre.ui, xi = pre.xi;
   int newly = 0;
   const float2 nxh = f2(-xi.x, -xi.y), nxl = f2(-xi.z, -xi.w), nuh = f2(-ui.x, -ui.y), nul = f2(-ui.z, -ui.w);
   const float2 ns2 = f2(-a.s2, -a.s2);
   float2 D1 = f2(0.f, 0.f), D2 = f2(0.f, 0.f), A = f2(0.f, 0.f);  // (d11, d12), (d21, d22), (ax, ay)
-  // 2 slots at a time: the halo walk reads shared memory, whose short latency needs less
-  // memory-level parallelism than global gathers did, and at 64 registers 4 blocks fit an
-  // SM (4-wide, 80 registers, 3 blocks: 61.4 us against 55.3 us on the 1M-particle plate)
-  walk_bonds<2>(w, 0, idx, gather, [&](int k, int j, const NbA& nb) {
-    const float2 e = tf_diff2(nb.x, nxh, nxl);  // xi^
-    const float2 d = tf_diff2(nb.u, nuh, nul);  // du^
-    if (BREAK) {  // d . (2 xi + d) - s2 xi . xi > 0, per component with one rounding
-      const float2 r = fma2(ns2, mul2(e, e), mul2(d, fma2(f2(2.f, 2.f), e, d)));
-      if (r.x + r.y > 0.f) {
-        const int64_t s = s0 + (int64_t)k * kChunk;
-        a.nbr[s] = -2 - a.nbr[s];  // the particle id of slot s (j may be a halo position)
-        if (a.loc) a.loc[s] = (uint16_t)pre.self_l;  // the slot now adds exact zeros
-        ++newly;
-        return;
+  // U bonds k .. k + U - 1, without a branch per bond: they are tested together,
+  // and where one breaks its du^ becomes zero, which adds exact zeros
+  auto bonds = [&](int k, auto u) {
+    constexpr int U = decltype(u)::value;
+    NbA nb[U];
+    float2 e[U], d[U];
+    float over[U], most = -1.f;
+    bool on[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int j = idx(k + q);
+      on[q] = Idx::kDense || j >= 0;
+      nb[q] = gather((int64_t)(on[q] ? j : 0));
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      e[q] = tf_diff2(nb[q].x, nxh, nxl);  // xi^
+      d[q] = tf_diff2(nb[q].u, nuh, nul);  // du^
+      if (!Idx::kDense && !on[q]) d[q] = f2(0.f, 0.f);
+      if (BREAK) {  // d . (2 xi + d) - s2 xi . xi > 0, per component with one rounding
+        const float2 r = fma2(ns2, mul2(e[q], e[q]), mul2(d[q], fma2(f2(2.f, 2.f), e[q], d[q])));
+        over[q] = !Idx::kDense && !on[q] ? -1.f : r.x + r.y;
+        most = fmaxf(most, over[q]);
       }
     }
-    if (UV) {
-      D1 = fma2(f2(d.x, d.x), e, D1);
-      D2 = fma2(f2(d.y, d.y), e, D2);
-      A = add2(A, d);
-    } else {
-      const float2 vv = f2(nb.v, nb.v);
-      const float2 t = mul2(vv, e);
-      D1 = fma2(f2(d.x, d.x), t, D1);
-      D2 = fma2(f2(d.y, d.y), t, D2);
-      A = fma2(vv, d, A);
+    if (BREAK && most > 0.f) {
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (over[q] > 0.f) {
+          const int64_t s = s0 + (int64_t)(k + q) * kChunk;
+          a.nbr[s] = -2 - a.nbr[s];
+          if (a.loc) a.loc[s] = (uint16_t)pre.self_l;  // the slot now adds exact zeros
+          ++newly;
+          d[q] = f2(0.f, 0.f);
+        }
     }
-  });
-  const float d11 = D1.x, d12 = D1.y, d21 = D2.x, d22 = D2.y;
-  a.hgs[p] = make_float2(2.f * a.k_hg * A.x, 2.f * a.k_hg * A.y);
-  float4 g = pre.geo;
-  int singular = pre.singular;
-  if (BREAK && newly) {
-    atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)newly);
-    const int64_t i = a.member[p];
-    const int32_t b = a.broken[i] + newly;
-    a.broken[i] = b;
-    a.damage[i] = (double)b / (double)a.fam[i];
-    kinv_update_mixed(a, i, p, s0, w);
-    g = a.geo[p];
-    singular = a.singular[p];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      if (UV) {
+        D1 = fma2(f2(d[q].x, d[q].x), e[q], D1);
+        D2 = fma2(f2(d[q].y, d[q].y), e[q], D2);
+        A = add2(A, d[q]);
+      } else {
+        const float2 vv = f2(nb[q].v, nb[q].v);
+        const float2 t = mul2(vv, e[q]);
+        D1 = fma2(f2(d[q].x, d[q].x), t, D1);
+        D2 = fma2(f2(d[q].y, d[q].y), t, D2);
+        A = fma2(vv, d[q], A);
+      }
+    }
+  };
+  // (at 64 registers 4 blocks fit an SM; a branch per bond kept a group's bonds from
+  // overlapping: 1M-particle plate, pass A 47.4 -> 45.4 us, and 58.3 -> 50.9 us with
+  // bonds breaking, of which ~4 us is the warp's K^-1 update)
+  if (live) {
+    int k = 0;
+    for (; k + kWalkA <= w; k += kWalkA) bonds(k, std::integral_constant<int, kWalkA>{});
+    for (; k < w; ++k) bonds(k, std::integral_constant<int, 1>{});
+    a.hgs[p] = make_float2(2.f * a.k_hg * A.x, 2.f * a.k_hg * A.y);
   }
-  if (singular) {
-    a.ws[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
+  if (live && newly == 0) a.ws[p] = pre.singular ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, D1, D2, pre.geo);
+  if (BREAK && __any_sync(0xffffffffu, newly != 0)) {
+    spare[threadIdx.x & 31] = make_float4(D1.x, D1.y, D2.x, D2.y);  // (the warp's staged indices are done with)
+    __syncwarp();
+    kinv_update_mixed_warp(a, p, s0, w, newly, spare);
   }
-  const float k11 = g.x, k12 = g.y, k22 = g.z, vi = g.w;
-  const float g11 = fmaf(d11, k11, d12 * k12), g12 = fmaf(d11, k12, d12 * k22);
-  const float g21 = fmaf(d21, k11, d22 * k12), g22 = fmaf(d21, k12, d22 * k22);
-  const float e11 = g11, e22 = g22, e12 = 0.5f * (g12 + g21);
-  const float s11 = fmaf(a.c11, e11, a.c12 * e22);
-  const float s22 = fmaf(a.c12, e11, a.c11 * e22);
-  const float s12 = a.c33 * e12;
-  const float kh = -a.k_hg;  // W^ = V^ (sigma^ K^-1 - k^ G), stored by columns {W11, W21, W12, W22}
-  a.ws[p] = make_float4(vi * fmaf(kh, g11, fmaf(s11, k11, s12 * k12)), vi * fmaf(kh, g21, fmaf(s12, k11, s22 * k12)),
-                        vi * fmaf(kh, g12, fmaf(s11, k12, s12 * k22)), vi * fmaf(kh, g22, fmaf(s12, k12, s22 * k22)));
 }
 
 struct GatherA {  // neighbour data of particle j (unstaged blocks)
@@ -315,7 +437,7 @@ __device__ __forceinline__ void pass_b_core(const MixedArgs& a, int64_t p, const
   // the rounding error of every addition into the next term
   float2 S = fma2(f2(wi.x, wi.y), f2(m.x, m.x), fma2(f2(wi.z, wi.w), f2(m.y, m.y), h)), C = f2(0.f, 0.f);
   const float2 nxh = f2(-xi.x, -xi.y), nxl = f2(-xi.z, -xi.w);
-  walk_bonds<4>(w, 0, idx, gather, [&](int, int, const NbB& nb) {
+  walk_bonds<kWalkB>(w, 0, idx, gather, [&](int, int, const NbB& nb) {
     const float2 e = tf_diff2(nb.x, nxh, nxl);
     const float2 p = fma2(f2(nb.w.x, nb.w.y), f2(e.x, e.x), mul2(f2(nb.w.z, nb.w.w), f2(e.y, e.y)));
     const float2 y = sub2(p, C);
@@ -484,7 +606,8 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
     if (w > 0 && lane == 0) stage_issue(mine, a.nbr + base, (uint32_t)w * 128u, &bars[warp]);
     __syncwarp();
     if (!warp_stage_done(a, &bars[warp], w)) return false;
-    if (live) pass_a_core<BREAK, UV>(a, p, pre, w, base + lane, SharedIdx{mine, lane}, GatherA{&a});
+    pass_a_core<BREAK, UV>(a, p, live, pre, w, base + lane, SharedIdx{mine, lane}, GatherA{&a},
+                           reinterpret_cast<float4*>(mine));
     return true;
   }
   const HaloSmem h = halo_smem(a, sm);
@@ -500,12 +623,12 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
   __syncthreads();
   if (!has) return true;
   if (!warp_stage_done(a, &bars[warp], w)) return false;
-  if (!live) return true;
   const float4* q0 = h.q0;
   const float4* q1 = h.q1;
   const float* vh = h.vh;
-  pass_a_core<BREAK, UV>(a, p, pre, w, base + lane, SharedHaloIdx{h.li + warp * a.wmax * 32, lane},
-                     [=](int64_t l) { return NbA{q0[l], q1[l], vh[l]}; });
+  pass_a_core<BREAK, UV>(a, p, live, pre, w, base + lane, SharedHaloIdx{h.li + warp * a.wmax * 32, lane},
+                     [=](int64_t l) { return NbA{q0[l], q1[l], UV ? 1.f : vh[l]}; },
+                         reinterpret_cast<float4*>(h.li + warp * a.wmax * 32));
   return true;
 }
 
