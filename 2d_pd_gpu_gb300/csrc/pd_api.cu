@@ -1654,6 +1654,81 @@ static cudaError_t enqueue_host_step_mixed(pd_ctx* c, int32_t nsteps, const doub
   return e;
 }
 
+// Below these sizes the slab pipelines' ~100 driver calls (0.15 - 0.25 ms) cost
+// more than the copies they hide: the import, and the last pass B's export, read
+// and write the page-locked buffers themselves, on one stream.  Per call, pipeline
+// against one stream, us: FP64, one step 100 x 100 213 / 65, 450 x 450 248 / 238,
+// 500 x 500 278 / 285, 1000 x 1000 814 / 974; mixed, one step 203 x 101 154 / 65,
+// 851 x 851 483 / 445, 1000 x 1000 537 / 554.
+constexpr int64_t kPipelineFrom = 220000, kPipelineFromMixed = 900000;
+
+// The graph of kInnerSteps steps between an import and the last step: pass A,
+// pass B + the next drift, each.  One per context (under the key -kInnerSteps of
+// its graphs), whatever the callers' step counts.
+constexpr int32_t kInnerSteps = 16;
+static int inner_graph(pd_ctx* c, cudaGraphExec_t* out) {
+  const auto it = c->graphs.find(-kInnerSteps);
+  if (it != c->graphs.end()) {
+    *out = it->second;
+    return PD_OK;
+  }
+  cudaGraph_t g;
+  PD_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  Launcher L(c);
+  for (int32_t k = 0; k < kInnerSteps; ++k) {
+    L.pass_a(c->stream);
+    L.pass_b(true, c->stream);
+  }
+  cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  if (e != cudaSuccess) return cuda_fail(c, e, "graph capture");
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return cuda_fail(c, e, "graph instantiate");
+  c->graphs.emplace(-kInnerSteps, *out);
+  return PD_OK;
+}
+
+// pd_step_host of a small plate; in, out: the buffers' device addresses.
+static int small_host_step(pd_ctx* c, int32_t nsteps, const double2* const in[3], double2* const out[3]) {
+  cudaStream_t s = c->stream;
+  const bool brk = c->p.s_c > 0.0;
+  Launcher L(c);
+  if (mixed(c)) {
+    pd::launch_import_drift_mixed(L.m, 0, L.m.nblocks, in[0], in[1], in[2], s);
+  } else {
+    Fp64Args z = L.f;
+    z.in_u = in[0];
+    z.in_v = in[1];
+    z.in_f = in[2];
+    pd::launch_drift_fp64(z, s);
+  }
+  int32_t left = nsteps - 1;
+  for (; left >= kInnerSteps; left -= kInnerSteps) {
+    cudaGraphExec_t ge = nullptr;
+    const int rc = inner_graph(c, &ge);
+    if (rc != PD_OK) return rc;
+    PD_CK(c, cudaGraphLaunch(ge, s));
+  }
+  for (; left > 0; --left) {
+    L.pass_a(s);
+    L.pass_b(true, s);
+  }
+  if (mixed(c)) {
+    pd::launch_slab_pass_a_mixed(L.m, brk, s);
+    L.m.out_u = out[0];
+    L.m.out_v = out[1];
+    L.m.out_f = out[2];
+    pd::launch_slab_pass_b_mixed(L.m, true, s);
+  } else {
+    pd::launch_pass_a_fp64(L.f, brk, s);
+    L.f.out_u = out[0];
+    L.f.out_v = out[1];
+    L.f.out_f = out[2];
+    pd::launch_pass_b_fp64(L.f, 0, s, true);
+  }
+  return PD_OK;
+}
+
 int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_in, const double* f_in, double* u_out,
                  double* v_out, double* f_out) {
   if (!c) return PD_ERR_ARG;
@@ -1666,9 +1741,22 @@ int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_
     if (!mapped_host(u_in) || !mapped_host(v_in) || !mapped_host(f_in) || !mapped_host(u_out) ||
         !mapped_host(v_out) || !mapped_host(f_out))
       return fail(c, PD_ERR_ARG, "pd_step_host: buffers must be page-locked host memory (pd_host_alloc)");
-    const int rp = plan_slabs_mixed(c);
-    if (rp != PD_OK) return rp;
-    PD_CK(c, enqueue_host_step_mixed(c, nsteps, u_in, v_in, f_in, u_out, v_out, f_out, c->p.s_c > 0.0));
+    if (c->n < kPipelineFromMixed) {
+      const double2* in[3];
+      double2* out[3];
+      const double* hin[3] = {u_in, v_in, f_in};
+      double* hout[3] = {u_out, v_out, f_out};
+      for (int k = 0; k < 3; ++k) {
+        in[k] = static_cast<const double2*>(mapped_host(hin[k]));
+        out[k] = static_cast<double2*>(mapped_host(hout[k]));
+      }
+      const int rs = small_host_step(c, nsteps, in, out);
+      if (rs != PD_OK) return rs;
+    } else {
+      const int rp = plan_slabs_mixed(c);
+      if (rp != PD_OK) return rp;
+      PD_CK(c, enqueue_host_step_mixed(c, nsteps, u_in, v_in, f_in, u_out, v_out, f_out, c->p.s_c > 0.0));
+    }
     PD_CK(c, cudaGetLastError());
     PD_CK(c, cudaStreamSynchronize(c->stream));
     c->steps += nsteps;
@@ -1693,6 +1781,11 @@ int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_
       pd::launch_ba_pass_a(plain, ba_args(c), s);
       pd::launch_ba_pass_b(last ? out : plain, ba_args(c), last ? 0 : 1, s);
     }
+  } else if (c->n < kPipelineFrom) {
+    const double2* from[3] = {in.in_u, in.in_v, in.in_f};
+    double2* to[3] = {out.out_u, out.out_v, out.out_f};
+    const int rs = small_host_step(c, nsteps, from, to);
+    if (rs != PD_OK) return rs;
   } else {
     const int rp = plan_slabs(c);
     if (rp != PD_OK) return rp;
@@ -1728,13 +1821,23 @@ int pd_compute_velocity(pd_ctx* c, const double* u, double* velocity, double* ac
     // page-locked buffers (pd_host_alloc): pd_step_host's slab pipeline, the
     // copies in overlapping pass A and each slab's pass B writing its results
     // back while later slabs compute; the same results as the staged call
-    const int rp = plan_slabs(c);
-    if (rp != PD_OK) return rp;
     Fp64Args out = fp64_args(c);
     out.out_v = static_cast<double2*>(mapped_host(velocity));
     out.out_a = static_cast<double2*>(mapped_host(acce));
     out.out_f = static_cast<double2*>(mapped_host(netF));
-    PD_CK(c, enqueue_host_step(c, 1, u, velocity, acce, fp64_args(c), out, c->p.s_c > 0.0, true));
+    if (c->n < kPipelineFrom) {  // (too small for the pipeline: one import of u, velocity and acce)
+      Fp64Args in = fp64_args(c);
+      in.in_u = static_cast<const double2*>(mapped_host(u));
+      in.in_v = out.out_v;
+      in.in_a = out.out_a;
+      pd::launch_shadow_fp64(in, s);
+      pd::launch_pass_a_fp64(fp64_args(c), c->p.s_c > 0.0, s);
+      pd::launch_pass_b_fp64(out, 2, s, true);
+    } else {
+      const int rp = plan_slabs(c);
+      if (rp != PD_OK) return rp;
+      PD_CK(c, enqueue_host_step(c, 1, u, velocity, acce, fp64_args(c), out, c->p.s_c > 0.0, true));
+    }
     PD_CK(c, cudaGetLastError());
     PD_CK(c, cudaStreamSynchronize(s));
     c->steps += 1;

@@ -220,8 +220,10 @@ int pd_step(pd_ctx* ctx, int32_t nsteps);
  * contexts: in one-step calls each slab's pass B writes its new state to
  * u_out, v_out, f_out directly over the CPU-GPU link while later slabs'
  * pass A runs (in longer calls, the last pass B does); mixed contexts the
- * same, through the mixed form's own slabs of spatial tiles.  In and out may
- * be the same buffers.
+ * same, through the mixed form's own slabs of spatial tiles.  Small plates
+ * (FP64 below 220,000 particles, mixed below 900,000) go without the slabs:
+ * the first kernel reads the buffers and the last one writes them.  In and
+ * out may be the same buffers.
  * Synchronous; the device state and the outputs are those of pd_set_state +
  * pd_step + pd_get_state, bit for bit. */
 int pd_step_host(pd_ctx* ctx, int32_t nsteps, const double* u_in, const double* v_in, const double* f_in,
@@ -239,9 +241,10 @@ int pd_synchronize(pd_ctx* ctx);
  * buffers stay allocated between calls.  The bond mask persists across calls
  * and breaks bonds as in pd_step when s_c > 0.  When all four buffers are
  * page-locked (pd_host_alloc) and the context is in the plain mode, the call
- * runs pd_step_host's slab pipeline: the copies in overlap the first pass,
- * and each slab's results go back while later slabs compute; the results are
- * the same bit for bit. */
+ * runs as pd_step_host's first and last step do: from 220,000 particles on its
+ * slab pipeline (the copies in overlap the first pass, and each slab's results
+ * go back while later slabs compute), below that the kernels read and write the
+ * buffers; the results are the same bit for bit. */
 int pd_compute_velocity(pd_ctx* ctx, const double* u, double* velocity, double* acce, double* netF);
 
 /* One FP64 force + kick, pd_compute_velocity's arithmetic, on CALLER-OWNED
