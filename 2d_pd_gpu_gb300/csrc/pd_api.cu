@@ -61,8 +61,9 @@ struct pd_ctx {
   double2* ba_ex = nullptr;  // exp(+-n1 |xi| / l)
   double2* ba_kq0 = nullptr;  // K_b^-1 with its det-guard flag
   double2* ba_kq1 = nullptr;
-  double* ba_wtri = nullptr;  // and, per particle, its weight matrix's lower triangle
+  double* ba_wfull = nullptr;  // and, per particle, its weight matrix
   double* ba_rv = nullptr;    // and 1 / its family's volume
+  bool mask_cut = false;      // bonds may have broken since the last reset (under earlier parameters)
   int32_t max_family = 0;
   // pd_step_host's copy / compute pipeline (streams and events, see plan_slabs)
   cudaStream_t io[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -200,7 +201,7 @@ void free_families(pd_ctx* c) {
   dfree(c->ba_ex);
   dfree(c->ba_kq0);
   dfree(c->ba_kq1);
-  dfree(c->ba_wtri);
+  dfree(c->ba_wfull);
   dfree(c->ba_rv);
   c->sell = pd::SellLayout{};
   c->slab_bnd.clear();
@@ -297,7 +298,8 @@ pd::BondAssoc ba_args(pd_ctx* c) {
   b.ex = c->ba_ex;
   b.kq0 = c->ba_kq0;
   b.kq1 = c->ba_kq1;
-  b.wtri = c->ba_wtri;
+  b.wfull = c->ba_wfull;
+  b.max_family = c->max_family;
   b.rv = c->ba_rv;
   return b;
 }
@@ -320,8 +322,8 @@ int ensure_ba(pd_ctx* c) {
   if (!c->ba_kq0) PD_CK(c, cudaMalloc(&c->ba_kq0, ns * sizeof(double2)));
   if (!c->ba_kq1) PD_CK(c, cudaMalloc(&c->ba_kq1, ns * sizeof(double2)));
   if (!c->ba_rv) PD_CK(c, cudaMalloc(&c->ba_rv, (size_t)(c->n > 0 ? c->n : 1) * sizeof(double)));
-  if (!c->ba_wtri)
-    PD_CK(c, cudaMalloc(&c->ba_wtri, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaTri * sizeof(double)));
+  if (!c->ba_wfull)
+    PD_CK(c, cudaMalloc(&c->ba_wfull, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaFull * sizeof(double)));
   pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
   if (!c->rslot) PD_CK(c, cudaMalloc(&c->rslot, ns * sizeof(int64_t)));
   PD_CK(c, cudaMalloc(&c->tb, ns * sizeof(double2)));
@@ -334,6 +336,14 @@ int ensure_ba(pd_ctx* c) {
   PD_CK(c, cudaStreamSynchronize(c->stream));
   if (err & pd::ERR_ASYMMETRIC) return fail(c, PD_ERR_ARG, "bond-associated mode needs symmetric families");
   return PD_OK;
+}
+
+// The bond-associated tables and reverse slots hold the families' intact bonds as they were
+// when they were formed: after a change of the mask (a reset or a restore) they are formed again.
+void reform_ba(pd_ctx* c) {
+  if (!bond_assoc(c) || !c->tb) return;
+  pd::launch_ba_reverse(fp64_args(c), ba_args(c), c->stream);
+  pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
 }
 
 bool mixed(const pd_ctx* c) { return c->p.precision == PD_MIXED; }
@@ -594,6 +604,7 @@ int pd_set_params(pd_ctx* c, const pd_params* p) {
   if (p->device != c->p.device || p->precision != c->p.precision)
     return fail(c, PD_ERR_ARG, "device and precision are fixed at pd_create");
   PD_CK(c, cudaSetDevice(c->p.device));
+  c->mask_cut = c->mask_cut || c->p.s_c > 0.0;
   c->p = *p;
   c->c_override = false;
   c->mz_table_ok = false;
@@ -800,9 +811,11 @@ int pd_reset(pd_ctx* c) {
     PD_CK(c, cudaMemsetAsync(c->hg, 0, nn * sizeof(double2), s));
     PD_CK(c, cudaMemsetAsync(c->u32, 0, nn * sizeof(float2), s));
     pd::launch_init_geometry_fp64(fp64_args(c), s);
+    if (c->mask_cut) reform_ba(c);
   }
   PD_CK(c, cudaGetLastError());
   PD_CK(c, cudaStreamSynchronize(s));
+  c->mask_cut = false;
   c->steps = 0;
   return PD_OK;
 }
@@ -1270,6 +1283,8 @@ int pd_checkpoint_load(pd_ctx* c, const void* buf, int64_t bytes) {
   } else {
     pd::launch_init_geometry_fp64(fp64_args(c), s);
     pd::launch_shadow_fp64(fp64_args(c), s);
+    reform_ba(c);
+    c->mask_cut = true;  // (the blob's mask may have broken bonds)
   }
   PD_CK(c, cudaGetLastError());
   PD_CK(c, cudaMemcpyAsync(c->counters, h.counters, sizeof(h.counters), cudaMemcpyHostToDevice, s));

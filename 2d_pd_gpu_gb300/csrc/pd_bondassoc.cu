@@ -19,14 +19,15 @@
 // formed once, at set-up and on every parameter change, by the set-up form of
 // pass A (k_ba_pass_a<true>, after k_ba_bonds): per slot |xi|, 1/|xi|,
 // exp(+-n1 |xi| / l) and K_b^-1 with its det-guard flag; per particle, 1 / V_h
-// and, with <= 32 bonds, the lower triangle of its weight matrix.
+// and, with <= 32 bonds, its weight matrix.
 //
 // Pass A runs one warp per particle and one lane per bond (families <= 64
 // bonds, two per lane): the family's bond data is staged in shared memory,
-// the weight triangle is loaded into a 32 x 32 matrix there, lane q sums D_q
-// over k in family order (the oracle's order) and forms V_q P_q, and, once
-// every P_b is in shared memory, lane j sums T_ij over b: 8 FP64 fma per
-// ordered pair of bonds.  A family of more than 32 bonds evaluates each lane's
+// lane q sums D_q over k in family order (the oracle's order) with its column of
+// the weight matrix and forms V_q P_q, and, once every P_b is in shared memory,
+// lane j sums T_ij over b: 8 FP64 fma per ordered pair of bonds.  Where no family
+// exceeds 32 bonds the column stays in the lane's registers (k_ba_pass_a_small);
+// else the matrix is loaded into shared memory (k_ba_pass_a<false>).  A family of more than 32 bonds evaluates each lane's
 // weight row inside its D_q loop and keeps the rows of the first 32 bonds.
 // The weight matrix is symmetric bit for bit (its products commute, and the
 // exponential factor is ordered by the two lengths), so only its lower
@@ -48,7 +49,7 @@ namespace pd {
 namespace {
 
 constexpr int kBaMax = 64;
-constexpr int kBaWarps = 2;  // particles per block of pass A (28 KB of shared memory per block: 7 per SM)
+constexpr int kBaWarps = 2;  // particles per block of pass A (k_ba_pass_a: 28 KB of shared memory, 7 blocks per SM)
 
 struct BaFamily {  // one particle's bonds, in family order
   double ex[kBaMax], ey[kBaMax], vv[kBaMax];
@@ -165,26 +166,25 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
   wf.direct = !(fabs(b.n1) * lmax * b.inv_wlen < 600.0);
   __syncwarp();
   const bool tri = n <= 32;
-  if (tri) {  // pair p = k (k + 1) / 2 + q, q <= k, of the lower triangle
-    // (the set-up form evaluates it and keeps it per particle; the step reads it back)
-    const int npair = n * (n + 1) / 2;
-    double* wt = b.wtri + i * kBaTri;
-    for (int p = lane; p < npair; p += 32) {
-      int k = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
-      if ((k + 1) * (k + 2) / 2 <= p) ++k;
-      if (k * (k + 1) / 2 > p) --k;
-      const int q = p - k * (k + 1) / 2;
-      double wqk;
-      if (KTAB) {
-        wqk = wf(F, q, k);
-        wt[p] = wqk;
-      } else {
-        wqk = wt[p];
+  if (tri) {
+    double* wt = b.wfull + i * kBaFull;
+    if (KTAB) {  // pair p = k (k + 1) / 2 + q, q <= k, of the lower triangle, evaluated and kept
+      const int npair = n * (n + 1) / 2;
+      for (int p = lane; p < npair; p += 32) {
+        int k = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
+        if ((k + 1) * (k + 2) / 2 <= p) ++k;
+        if (k * (k + 1) / 2 > p) --k;
+        const int q = p - k * (k + 1) / 2;
+        const double wqk = wf(F, q, k);
+        F.wrow[k][q] = wqk;
+        F.wrow[q][k] = wqk;
       }
-      F.wrow[k][q] = wqk;
-      F.wrow[q][k] = wqk;
+      __syncwarp();
+      for (int k = 0; k < 32; ++k) wt[k * 32 + lane] = k < n && lane < n ? F.wrow[k][lane] : 0.0;
+    } else {
+      for (int k = 0; k < n; ++k) F.wrow[k][lane] = wt[k * 32 + lane];
+      __syncwarp();
     }
-    __syncwarp();
   }
   // P_b = sigma_b K_b^-1 of bond q (KTAB: K_b^-1)
   for (int q = lane; q < n; q += 32) {
@@ -257,6 +257,111 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
     }
     const double ex = F.ex[jj], ey = F.ey[jj];
     b.tb[F.slot[jj]] = make_double2(fma(m11 * rv, ex, (m12 * rv) * ey), fma(m21 * rv, ex, (m22 * rv) * ey));
+  }
+}
+
+// The step's pass A where no family exceeds 32 bonds: k_ba_pass_a's operations
+// in the same order, with lane q's column of the weight matrix in its registers:
+// the 28 loads of a column are requested together at the start, ahead of the
+// staging, and serve both sums, and 3.1 KB of shared memory per warp instead of
+// 14 let ~20 warps share an SM instead of 14.  Step of the 70 x 60 mesh 78 -> 70 us
+// (its FP64 operations alone take 59), 20 x 20 23.6 -> 18.6, 90 x 90 137 -> 127.
+struct BaSmall {
+  double S[32][4], P[32][4];  // V_k d_k (x) xi_k; V_b sigma_b K_b^-1
+  double2 e[32];
+  double vv[32];
+  int64_t slot[32];
+};
+
+__global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a_small(Fp64Args a, BondAssoc b) {
+  __shared__ BaSmall fam[kBaWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i = (int64_t)blockIdx.x * kBaWarps + warp;
+  if (i >= a.n) return;  // warp-uniform
+  BaSmall& F = fam[warp];
+  const int64_t c0 = i >> 5;
+  const int w = a.chunk_w[c0];
+  const int64_t s = a.chunk_base[c0] + (i & 31) + (int64_t)lane * kChunk;
+  const double* wt = b.wfull + i * kBaFull + lane;
+  const int j = lane < w ? a.nbr[s] : -1;
+  double wk[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) wk[k] = k < w ? wt[k * 32] : 0.0;
+  const double2 ui = a.u[i];
+  const double rv = b.rv[i];
+  const unsigned m = __ballot_sync(0xffffffffu, j >= 0);
+  const int n = __popc(m);
+  if (j >= 0) {
+    const int q = __popc(m & ((1u << lane) - 1u));
+    const double2 e = a.bxi[s], uj = a.u[j];
+    const double vj = a.vol[j];
+    const double t0 = vj * e.x, t1 = vj * e.y;
+    const double dx = uj.x - ui.x, dy = uj.y - ui.y;
+    F.S[q][0] = dx * t0;
+    F.S[q][1] = dx * t1;
+    F.S[q][2] = dy * t0;
+    F.S[q][3] = dy * t1;
+    F.e[q] = e;
+    F.vv[q] = vj;
+    F.slot[q] = s;
+  }
+  // (the sums run by groups of four: an operation that is predicated off keeps the FP64 pipe
+  // busy all the same, so only the last group's rest is padding, whose zeros add exactly)
+  if (lane >= n && lane < ((n + 3) & ~3))
+    F.S[lane][0] = F.S[lane][1] = F.S[lane][2] = F.S[lane][3] = F.P[lane][0] = F.P[lane][1] = F.P[lane][2] = F.P[lane][3] = 0.0;
+  __syncwarp();
+  const int64_t sl = lane < n ? F.slot[lane] : 0;
+  double2 kq0 = make_double2(0.0, 0.0), kq1 = make_double2(0.0, 1.0);
+  if (lane < n) {
+    kq0 = b.kq0[sl];
+    kq1 = b.kq1[sl];
+  }
+  double d11 = 0.0, d12 = 0.0, d21 = 0.0, d22 = 0.0;
+#pragma unroll
+  for (int k0 = 0; k0 < 32; k0 += 4) {
+    if (k0 >= n) break;
+#pragma unroll
+    for (int k = k0; k < k0 + 4; ++k) {
+      d11 = fma(wk[k], F.S[k][0], d11);
+      d12 = fma(wk[k], F.S[k][1], d12);
+      d21 = fma(wk[k], F.S[k][2], d21);
+      d22 = fma(wk[k], F.S[k][3], d22);
+    }
+  }
+  if (lane < n) {
+    if (__double_as_longlong(kq1.y) != 0) {  // K_b failed the det guard
+      F.P[lane][0] = F.P[lane][1] = F.P[lane][2] = F.P[lane][3] = 0.0;
+    } else {
+      const double q11 = kq0.x, q12 = kq0.y, q22 = kq1.x;
+      const double g11 = fma(d11, q11, d12 * q12), g12 = fma(d11, q12, d12 * q22);
+      const double g21 = fma(d21, q11, d22 * q12), g22 = fma(d21, q12, d22 * q22);
+      const double e11 = g11, e22 = g22, e12 = 0.5 * (g12 + g21);
+      const double s11 = fma(a.c11, e11, a.c12 * e22);
+      const double s22 = fma(a.c12, e11, a.c11 * e22);
+      const double s12 = a.c33 * e12;
+      const double vq = F.vv[lane];
+      F.P[lane][0] = vq * fma(s11, q11, s12 * q12);
+      F.P[lane][1] = vq * fma(s11, q12, s12 * q22);
+      F.P[lane][2] = vq * fma(s12, q11, s22 * q12);
+      F.P[lane][3] = vq * fma(s12, q12, s22 * q22);
+    }
+  }
+  __syncwarp();
+  double m11 = 0.0, m12 = 0.0, m21 = 0.0, m22 = 0.0;
+#pragma unroll
+  for (int k0 = 0; k0 < 32; k0 += 4) {
+    if (k0 >= n) break;
+#pragma unroll
+    for (int k = k0; k < k0 + 4; ++k) {
+      m11 = fma(wk[k], F.P[k][0], m11);
+      m12 = fma(wk[k], F.P[k][1], m12);
+      m21 = fma(wk[k], F.P[k][2], m21);
+      m22 = fma(wk[k], F.P[k][3], m22);
+    }
+  }
+  if (lane < n) {
+    const double2 e = F.e[lane];
+    b.tb[sl] = make_double2(fma(m11 * rv, e.x, (m12 * rv) * e.y), fma(m21 * rv, e.x, (m22 * rv) * e.y));
   }
 }
 
@@ -379,7 +484,12 @@ void launch_ba_bonds(const Fp64Args& a, const BondAssoc& b, int64_t nslots, cuda
 }
 
 void launch_ba_pass_a(const Fp64Args& a, const BondAssoc& b, cudaStream_t s) {
-  if (a.n > 0) k_ba_pass_a<false><<<(unsigned)((a.n + kBaWarps - 1) / kBaWarps), 32 * kBaWarps, 0, s>>>(a, b);
+  if (a.n <= 0) return;
+  const unsigned nb = (unsigned)((a.n + kBaWarps - 1) / kBaWarps);
+  if (b.max_family <= 32)
+    k_ba_pass_a_small<<<nb, 32 * kBaWarps, 0, s>>>(a, b);
+  else
+    k_ba_pass_a<false><<<nb, 32 * kBaWarps, 0, s>>>(a, b);
 }
 
 void launch_ba_pass_b(const Fp64Args& a, const BondAssoc& b, int mode, cudaStream_t s) {

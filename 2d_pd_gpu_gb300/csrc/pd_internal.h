@@ -117,10 +117,11 @@ struct BondAssoc {
   double2* ex;     // per bond slot: exp(n1 |xi| / l), exp(-n1 |xi| / l) (for the weights n1, l of the call)
   double2* kq0;    // per bond slot: K_b^-1 (q11, q12)
   double2* kq1;    // per bond slot: (q22, 1 if K_b fails the det guard else 0)
-  double* wtri;    // per particle with <= 32 bonds: its weight matrix's lower triangle (kBaTri doubles)
+  double* wfull;   // per particle with <= 32 bonds: its weight matrix, w(q, k) at [k][q] (kBaFull doubles)
   double* rv;      // per particle: 1 / its family's volume
+  int32_t max_family, pad;
 };
-constexpr int64_t kBaTri = 32 * 33 / 2;
+constexpr int64_t kBaFull = 32 * 32;
 
 // Mazars damage (pd_mazars.cu): law constants and per-slot history.
 struct MazarsArgs {
