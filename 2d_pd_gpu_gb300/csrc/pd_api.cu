@@ -1294,44 +1294,43 @@ int pd_checkpoint_load(pd_ctx* c, const void* buf, int64_t bytes) {
 }
 
 
-// pd_step_host pipeline (FP64 form).  The particles are cut into kSlabs index
-// ranges (multiples of 32): 1/64 and 3/64 of the plate, six of 1/8, then 3/32,
-// 1/16 and 1/32, so the first pass A starts after a few microseconds of
-// copying, the later copies stay ahead of it, and the last slabs, whose pass
-// B and write-back end the call, are short (1M-particle plate, ms per one-step
-// call: these slabs 0.844-0.848 against 0.864-0.887 for seven of 1/8 after the
-// same two; 1/128, 1/128, 1/64, 1/32, 1/16, then seven of 1/8 0.862; 1/32,
-// 3/32, 1/8, then four of 3/16 0.862; five of 3/16 after 1/16 0.874; trailing
-// 1/16, 1/16, 1/32, 1/64, 1/64 or 3/32, 3/32, 1/16, 1/32, 1/32 0.857-0.866);
+// pd_step_host pipeline (FP64 form).  The particles are cut into index ranges
+// (slabs, multiples of 32), the first and the last ones short, so the first pass A
+// starts after a few microseconds of copying, the copies stay ahead of it, and the
+// slabs whose pass B and write-back end the call are brief.  From kFineSlabsFrom
+// particles on the even slabs between them hold about 62,000 particles each: fewer,
+// and their passes A leave SMs idle; more, and less of a slab's copies and write-back
+// runs under other slabs' passes (us per one-step call, 1M particles: 8 slabs 864,
+// 11 818, 14 806, 16 797, 19 790, 20 788).  Below, 11 slabs: more of them only cost
+// launches (us: 360,000 particles: 11 slabs 347, 14 348, 19 356; 624,000: 11 slabs
+// 537, 14 545; 810,000: 11 slabs 675, 16 665).
 // slab_need[k] / slab_low[k] = the last / first slab holding a neighbour of
 // slab k's particles.  Streams (io[0], io[1] at high priority): io[1] copies
 // u, v, f in slab by slab, io[0] runs each slab's drift as its copy lands (the
 // first kZeroCopySlabs slabs' drifts read the input buffers directly),
-// pass A of slab k starts on its own stream once slabs 0 .. slab_need[k] are
-// in, and, in one-step calls, pass B of slab k (its own stream) once pass A
-// of slabs slab_low[k] .. slab_need[k] is done, writing the slab's new state
-// straight to the host buffers -- so the device-to-host traffic runs under
-// the later slabs' pass A instead of after it.  One stream per launch: an
-// FP64 pass A block runs for ~70 us whatever the slab's size (one thread per
-// particle, FP64-latency bound when the SM is not full), so slab launches
-// queued on shared streams would wait out each other's tails.
-constexpr int kSlabs = 11;
+// pass A of slab k starts once slabs 0 .. slab_need[k] are in, and, in one-step
+// calls, pass B of slab k once pass A of slabs slab_low[k] .. slab_need[k] is
+// done, writing the slab's new state straight to the host buffers -- so the
+// device-to-host traffic runs under the later slabs' pass A instead of after it.
+// The passes take kPassStreams streams each in turn: launches on one stream would
+// wait out each other's tails.
+constexpr int64_t kFineSlabsFrom = 700000, kEvenSlab = 62000;
+constexpr int kEvenMin = 6, kEvenMax = 13;
 // the first slabs are imported by their drift kernel reading the page-locked input directly
 // (no copy-engine start-up before the first pass A can begin: 0.852-0.855 -> 0.843-0.846 ms
 // per one-step call on the 1M-particle plate); the rest by copy engine
 constexpr int kZeroCopySlabs = 2;
+constexpr int kMaxSlabs = 6 + kEvenMax;  // the most slabs either form's pipeline uses
+constexpr int kPassStreams = 8;
 enum {
   kEvImport = 0,
-  kEvCopy = kSlabs,
-  kEvA = 2 * kSlabs,
-  kEvB = 3 * kSlabs,
-  kEvStart = 4 * kSlabs,
-  kEvJoin = 4 * kSlabs + 1,
-  kEvCount = 4 * kSlabs + 2
+  kEvCopy = kMaxSlabs,
+  kEvA = 2 * kMaxSlabs,
+  kEvB = 3 * kMaxSlabs,
+  kEvStart = 4 * kMaxSlabs,
+  kEvJoin = 4 * kMaxSlabs + 1,
+  kEvCount = 4 * kMaxSlabs + 2
 };
-
-constexpr int kMaxSlabs = 16;  // the most slabs either form's pipeline uses
-static_assert(kSlabs <= kMaxSlabs, "one pass stream pair per slab");
 
 // The pipeline's streams (io[0], io[1], io[5] at high priority; the per-slab
 // pass streams at low priority) and events.
@@ -1341,7 +1340,7 @@ static int pipeline_streams(pd_ctx* c, int nev) {
     PD_CK(c, cudaDeviceGetStreamPriorityRange(&lo, &hi));
     for (int q = 0; q < 6; ++q)
       PD_CK(c, cudaStreamCreateWithPriority(&c->io[q], cudaStreamNonBlocking, q < 2 || q == 5 ? hi : lo));
-    while ((int)c->ps.size() < 2 * kMaxSlabs) {
+    while ((int)c->ps.size() < 2 * kPassStreams) {
       cudaStream_t q;
       PD_CK(c, cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, lo));
       c->ps.push_back(q);
@@ -1375,26 +1374,35 @@ static int plan_slabs(pd_ctx* c) {
     e = copy_sync(hl.data(), reach + nch, hl.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
   cudaFree(reach);
   PD_CK(c, e);
-  // slab boundaries in chunks: 1/64, 3/64, six of 1/8, then 3/32, 1/16, 1/32
-  static const int kShare[kSlabs] = {4, 12, 32, 32, 32, 32, 32, 32, 24, 16, 8};  // of 256
-  std::vector<int64_t> bc(kSlabs + 1, 0);
-  int acc = 0;
-  for (int k = 0; k < kSlabs; ++k) {
-    acc += kShare[k];
-    bc[k + 1] = k + 1 == kSlabs ? nch : std::min<int64_t>(nch, std::max<int64_t>(bc[k] + 1, nch * acc / 256));
+  // slab boundaries in chunks
+  const bool fine = c->n >= kFineSlabsFrom;
+  const int even =
+      fine ? (int)std::min<int64_t>(kEvenMax, std::max<int64_t>(kEvenMin, c->n * 208 / 256 / kEvenSlab)) : kEvenMin;
+  std::vector<int64_t> share = fine ? std::vector<int64_t>{4, 8, 12} : std::vector<int64_t>{4, 12};  // of 256
+  const std::vector<int64_t> tail = fine ? std::vector<int64_t>{12, 8, 4} : std::vector<int64_t>{24, 16, 8};
+  const int64_t middle = fine ? 208 : 192;
+  for (int64_t& q : share) q *= even;  // now of 256 * even
+  share.insert(share.end(), (size_t)even, middle);
+  for (int64_t q : tail) share.push_back(q * even);
+  const int slabs = (int)share.size();
+  std::vector<int64_t> bc(slabs + 1, 0);
+  int64_t end = 0;
+  for (int k = 0; k < slabs; ++k) {
+    end += share[k];
+    bc[k + 1] = k + 1 == slabs ? nch : std::min<int64_t>(nch, std::max<int64_t>(bc[k] + 1, nch * end / (256 * even)));
   }
-  c->slab_bnd.assign(kSlabs + 1, 0);
-  for (int k = 0; k <= kSlabs; ++k) c->slab_bnd[k] = std::min<int64_t>(c->n, bc[k] * 32);
-  c->slab_need.assign(kSlabs, 0);
-  c->slab_low.assign(kSlabs, 0);
-  for (int k = 0; k < kSlabs; ++k) {
+  c->slab_bnd.assign(slabs + 1, 0);
+  for (int k = 0; k <= slabs; ++k) c->slab_bnd[k] = std::min<int64_t>(c->n, bc[k] * 32);
+  c->slab_need.assign(slabs, 0);
+  c->slab_low.assign(slabs, 0);
+  for (int k = 0; k < slabs; ++k) {
     int64_t far = -1, near = INT64_MAX;
     for (int64_t q = bc[k]; q < bc[k + 1]; ++q) {
       far = std::max<int64_t>(far, h[(size_t)q]);
       near = std::min<int64_t>(near, hl[(size_t)q]);
     }
     int need = k, low = k;
-    while (need + 1 < kSlabs && far >= c->slab_bnd[need + 1]) ++need;
+    while (need + 1 < slabs && far >= c->slab_bnd[need + 1]) ++need;
     while (low > 0 && near < c->slab_bnd[low]) --low;
     c->slab_need[k] = need;
     c->slab_low[k] = low;
@@ -1429,14 +1437,15 @@ static cudaError_t enqueue_host_step(pd_ctx* c, int32_t nsteps, const double* u_
   const size_t b16 = sizeof(double2);
   ck(cudaEventRecord(ev[kEvStart], s));
   for (int q = 0; q < 2; ++q) ck(cudaStreamWaitEvent(io[q], ev[kEvStart], 0));
-  cudaStream_t* pa = c->ps.data();           // pass A of slab k: pa[k]
-  cudaStream_t* pb = c->ps.data() + kMaxSlabs;  // pass B of slab k: pb[k]
+  const int slabs = (int)c->slab_need.size();
+  cudaStream_t* pa = c->ps.data();                 // pass A of slab k: pa[k % kPassStreams]
+  cudaStream_t* pb = c->ps.data() + kPassStreams;  // pass B alike
   // enqueued in dependency order (each pass A right after the import it waits for, each
   // pass B right after the last pass A it waits for), so the first pass A is submitted
   // before the host has issued the later imports
   const bool one = nsteps == 1;
   int next_a = 0, next_b = 0;
-  for (int k = 0; k < kSlabs; ++k) {
+  for (int k = 0; k < slabs; ++k) {
     const Fp64Args a = slab_args(c, plain, k);  // import slab k
     const size_t off = (size_t)a.i0, cnt = (size_t)(a.n - a.i0);
     if (k < kZeroCopySlabs) {  // the import kernel reads the page-locked input itself
@@ -1465,29 +1474,29 @@ static cudaError_t enqueue_host_step(pd_ctx* c, int32_t nsteps, const double* u_
         pd::launch_drift_fp64(a, io[0]);  // in place, on the device copy
     }
     ck(cudaEventRecord(ev[kEvImport + k], io[0]));
-    for (; next_a < kSlabs && c->slab_need[next_a] <= k; ++next_a) {  // pass A of slabs whose neighbours are in
-      cudaStream_t sj = pa[next_a];
+    for (; next_a < slabs && c->slab_need[next_a] <= k; ++next_a) {  // pass A of slabs whose neighbours are in
+      cudaStream_t sj = pa[next_a % kPassStreams];
       ck(cudaStreamWaitEvent(sj, ev[kEvImport + c->slab_need[next_a]], 0));  // (after the call's start)
       pd::launch_pass_a_fp64(slab_args(c, plain, next_a), brk, sj);
       ck(cudaEventRecord(ev[kEvA + next_a], sj));
       // one-step calls: pass B (with the write-back) of every slab whose neighbours' pass A is in
-      for (; one && next_b < kSlabs && c->slab_need[next_b] <= next_a; ++next_b) {
-        cudaStream_t sb = pb[next_b];
+      for (; one && next_b < slabs && c->slab_need[next_b] <= next_a; ++next_b) {
+        cudaStream_t sb = pb[next_b % kPassStreams];
         for (int q = c->slab_low[next_b]; q <= c->slab_need[next_b]; ++q) ck(cudaStreamWaitEvent(sb, ev[kEvA + q], 0));
         pd::launch_pass_b_fp64(slab_args(c, out, next_b), dropin ? 2 : 0, sb);
         ck(cudaEventRecord(ev[kEvB + next_b], sb));
       }
     }
   }
-  if (one && next_b != kSlabs) e = e == cudaSuccess ? cudaErrorLaunchFailure : e;  // (a plan bug)
+  if (one && next_b != slabs) e = e == cudaSuccess ? cudaErrorLaunchFailure : e;  // (a plan bug)
   // join every stream's work on the main stream
   auto join = [&](cudaStream_t q) {
     ck(cudaEventRecord(ev[kEvJoin], q));
     ck(cudaStreamWaitEvent(s, ev[kEvJoin], 0));
   };
   join(io[0]);
-  for (int k = 0; k < kSlabs; ++k) join(pa[k]);
-  for (int k = 0; one && k < kSlabs; ++k) join(pb[k]);
+  for (int k = 0; k < kPassStreams; ++k) join(pa[k]);
+  for (int k = 0; one && k < kPassStreams; ++k) join(pb[k]);
   if (!one)
     for (int32_t k = 0; k < nsteps; ++k) {
       const bool last = k + 1 == nsteps;
@@ -1529,7 +1538,7 @@ static cudaError_t enqueue_host_step(pd_ctx* c, int32_t nsteps, const double* u_
 // the input and output buffers the same, slab k's pass B overwrites only ids
 // of id slabs 0 .. k, whose copies in are complete before its import.
 constexpr int kMixedSlabs = 8;
-static_assert(kMixedSlabs <= kMaxSlabs, "one pass stream pair per slab");
+static_assert(kMixedSlabs <= kPassStreams, "one pass stream pair per slab");
 enum { kMEvIn = 0, kMEvImport = kMixedSlabs, kMEvA = 2 * kMixedSlabs, kMEvB = 3 * kMixedSlabs,
        kMEvStart = 4 * kMixedSlabs, kMEvCount = 4 * kMixedSlabs + 1 };
 
@@ -1613,7 +1622,7 @@ static cudaError_t enqueue_host_step_mixed(pd_ctx* c, int32_t nsteps, const doub
   ck(cudaEventRecord(ev[kMEvStart], s));
   for (int q = 0; q < 6; ++q) ck(cudaStreamWaitEvent(io[q], ev[kMEvStart], 0));
   cudaStream_t* pa = c->ps.data();           // pass A of slab k: pa[k]
-  cudaStream_t* pb = c->ps.data() + kMaxSlabs;  // pass B of slab k: pb[k]
+  cudaStream_t* pb = c->ps.data() + kPassStreams;  // pass B of slab k: pb[k]
   const bool one = nsteps == 1;
   int next_a = 0, next_b = 0;
   for (int k = 0; k < K; ++k) {  // enqueued in dependency order

@@ -64,3 +64,35 @@ def test_compute_velocity_routes_equal_pageable(pdg, nx, ny):
         assert np.array_equal(v, hv) and np.array_equal(acc, ha) and np.array_equal(fa, hf)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(837, 836), (837, 837), (1013, 991)])
+def test_slab_plans_equal_staged_steps(pdg, nx, ny):
+    """Either side of 700,000 particles, where the even slabs get finer, and the most slabs."""
+    test_step_host_routes_equal_staged_steps(pdg, False, nx, ny, (1, 3))
+
+
+@pytest.mark.parametrize("nx,ny,order", [(480, 480, "reversed"), (480, 480, "shuffled"), (840, 840, "reversed"),
+                                         (840, 840, "shuffled")])
+def test_slab_plans_other_numberings(pdg, nx, ny, order):
+    """Numberings in which the slabs' neighbours lie in earlier, or in all, slabs."""
+    import dataclasses
+    p = pdg.plates.make_plate(nx, ny, seed=9, crack="centre-half")
+    perm = np.arange(p.n)[::-1] if order == "reversed" else np.random.default_rng(2).permutation(p.n)
+    p = dataclasses.replace(p, x=np.ascontiguousarray(p.x[perm]), vol=np.ascontiguousarray(p.vol[perm]),
+                            group_of=np.ascontiguousarray(p.group_of[perm]))
+    a, b = p.context(), p.context()
+    bufs = [nat.PinnedArray((p.n, 2)) for nat in [pdg.native] * 3]
+    h = [x.array for x in bufs]
+    for seed, steps in enumerate((1, 2, 1)):
+        state = _state(p, seed)
+        for x, y in zip(h, state):
+            x[:] = y
+        a.set_state(*state)
+        a.step(steps)
+        b.step_host(steps, *h)
+        for w, x in zip(a.state(), h):
+            assert np.array_equal(w, x), steps
+    assert a.counters()["bonds_broken"] == b.counters()["bonds_broken"] > 0
+    a.close()
+    b.close()
