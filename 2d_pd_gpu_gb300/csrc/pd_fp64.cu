@@ -2,10 +2,10 @@
 // only fused multiply-adds are the explicit fma() calls, written in the same
 // places as the oracle's restatement, so results are bit-identical to it.
 //
-// One thread per particle, bonds walked in family order through the SELL-32
-// layout (every slot load of a warp is one coalesced line).  Per-particle sums
-// are sequential in family order, with no atomics, so results are
-// deterministic and independent of the launch shape.
+// Two threads per particle (one per component), bonds walked in family order
+// through the SELL-32 layout (a warp's slot loads are half a line each).
+// Per-particle sums are sequential in family order, with no atomics, so results
+// are deterministic and independent of the launch shape.
 //
 // Reference correspondence (src/main_seq.cpp):
 //   k_drift / pass B tail : applyVelocityBC :28-36, updatePositions :386-393,
@@ -97,8 +97,7 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
 // 1 / V, damage) and lanes 0 .. 4 one product; kinv_update's operations
 // (x + t is fma(t, 1, x)).  One thread alone has a chain of ~240 dependent FP64
 // operations here instead of ~45, each of which waits for its turn on the pipe,
-// and its pass waits for it (300 x 300 plate with bonds breaking, pass A:
-// 87 us against 72).
+// and its pass waits for it.
 __device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int64_t s0, int w, int newly) {
   const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
   unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
@@ -224,7 +223,8 @@ __global__ void __launch_bounds__(kBlock) k_shadow(Fp64Args a) {
 // could underflow or overflow, and any infinity or NaN, leave it to FP64.
 // A test that bounds |d| alone leaves every rotating or compressed bond to FP64
 // too, which in the few warps of a fracture zone is what the whole pass waits
-// for (300 x 300 plate with bonds breaking: see k_pass_a).
+// for (step with bonds breaking, 300 x 300 particles: 83 against 76 us; 200 x 200:
+// 43 against 33).
 __device__ __forceinline__ int stretch_fp32(float2 ui, float2 uj, float2 e, float s2) {
   const float fx = uj.x - ui.x, fy = uj.y - ui.y;
   const float dx = 6.0e-8f * (fabsf(uj.x) + fabsf(ui.x) + fabsf(fx));

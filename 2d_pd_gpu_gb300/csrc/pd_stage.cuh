@@ -63,15 +63,6 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
   return false;
 }
 
-// Warp-cooperative: copies src[0 .. 32 w) int32 (global) to dst (shared).
-// All 32 lanes call it.  False if the copy did not land in time.
-__device__ __forceinline__ bool stage_chunk(int32_t* dst, const int32_t* src, int w, uint64_t* bar) {
-  if (w <= 0) return true;
-  if ((threadIdx.x & 31u) == 0) stage_issue(dst, src, (uint32_t)w * 128u, bar);
-  __syncwarp();
-  return stage_wait(bar);
-}
-
 // Index of slot k of lane `lane` in a staged int32 chunk.
 struct SharedIdx {
   static constexpr bool kDense = false;

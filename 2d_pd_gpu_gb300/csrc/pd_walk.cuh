@@ -9,8 +9,8 @@
 // flight.  The body order is the sequential slot order, so sums are
 // bit-identical to the one-slot-at-a-time loop.
 //
-// idx(k) returns the neighbour index of the particle's slot k (from global
-// memory or from a staged shared-memory copy); body(k, j, g) gets the slot
+// idx(k) returns the neighbour index of the particle's slot k (from a staged
+// shared-memory copy); body(k, j, g) gets the slot
 // number k, the index j >= 0 and the gathered data.  An index source with
 // kDense = true never yields a negative index (padding and broken slots
 // point at data that contributes exact zeros), so the bodies run unguarded.
@@ -57,13 +57,5 @@ __device__ __forceinline__ void walk_bonds(int w, int64_t self, Idx idx, Gather 
     if (Idx::kDense || jj >= 0) body(k, jj, gather((int64_t)jj));
   }
 }
-
-// Streaming (evict-first) load of global slot s0 + 32 k of a SELL-32 row.
-struct GlobalIdx {
-  static constexpr bool kDense = false;
-  const int32_t* nbr;
-  int64_t s0;
-  __device__ __forceinline__ int operator()(int k) const { return __ldcs(&nbr[s0 + (int64_t)k * 32]); }
-};
 
 }  // namespace pd
