@@ -2,10 +2,10 @@
 // only fused multiply-adds are the explicit fma() calls, written in the same
 // places as the oracle's restatement, so results are bit-identical to it.
 //
-// Two threads per particle (one per component), bonds walked in family order
-// through the SELL-32 layout (a warp's slot loads are half a line each).
-// Per-particle sums are sequential in family order, with no atomics, so results
-// are deterministic and independent of the launch shape.
+// One thread per particle, bonds walked in family order through the SELL-32
+// layout (every slot load of a warp is one coalesced line).  Per-particle sums
+// are sequential in family order, with no atomics, so results are
+// deterministic and independent of the launch shape.
 //
 // Reference correspondence (src/main_seq.cpp):
 //   k_drift / pass B tail : applyVelocityBC :28-36, updatePositions :386-393,
@@ -36,9 +36,16 @@ __device__ __forceinline__ int64_t slot0(const Fp64Args& a, int64_t i, int* w) {
 // plate over the chip (200 x 200, per step: 43 us against 47 with 128 threads
 // and 72 with 256) and end a large one evenly.
 constexpr int kPairBlock = 64;
-// Bonds in flight per thread (pass A 1, 2, 4: 22.6, 18.7, 19.0 us per step of
-// a 100 x 100 plate; pass B 2, 4: 21.6, 18.7).
-constexpr int kWalkA = 2, kWalkB = 4;
+// Bonds per group of the passes' walks, two groups in flight (step with bonds
+// breaking, us, pass A 1, 2, 3 bonds: 100 x 100 particles 16.8, 16.3, 16.2, 1M 686,
+// 685, 711; pass B 2, 4: 1M 685, 710).
+constexpr int kWalkA = 2, kWalkB = 2;
+// Up to this many particles a pass lets the next one launch at its blocks' exit
+// only: launched while some SMs still hold blocks of this pass, the next one's
+// blocks crowd onto the others, and all of them fit at once, so nothing evens that
+// out (step, us: 150 x 150 particles 23.6 -> 20.0, 170 x 170 31.4 -> 22.9, with bonds
+// breaking 34 -> 23.6; 220 x 220 41.4 -> 37.0; 1M 686.4 against 687.3).
+constexpr int64_t kExitTrigger = 60000;
 
 // The passes run two threads per particle: thread h = 0 sums the x components
 // (d11, d12, the penalty's x; f.x), h = 1 the y components.  Every sum keeps
@@ -97,7 +104,8 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
 // 1 / V, damage) and lanes 0 .. 4 one product; kinv_update's operations
 // (x + t is fma(t, 1, x)).  One thread alone has a chain of ~240 dependent FP64
 // operations here instead of ~45, each of which waits for its turn on the pipe,
-// and its pass waits for it.
+// and its pass waits for it (300 x 300 plate with bonds breaking, pass A:
+// 87 us against 72).
 __device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int64_t s0, int w, int newly) {
   const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
   unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
@@ -223,8 +231,7 @@ __global__ void __launch_bounds__(kBlock) k_shadow(Fp64Args a) {
 // could underflow or overflow, and any infinity or NaN, leave it to FP64.
 // A test that bounds |d| alone leaves every rotating or compressed bond to FP64
 // too, which in the few warps of a fracture zone is what the whole pass waits
-// for (step with bonds breaking, 300 x 300 particles: 83 against 76 us; 200 x 200:
-// 43 against 33).
+// for (300 x 300 plate with bonds breaking: see k_pass_a).
 __device__ __forceinline__ int stretch_fp32(float2 ui, float2 uj, float2 e, float s2) {
   const float fx = uj.x - ui.x, fy = uj.y - ui.y;
   const float dx = 6.0e-8f * (fabsf(uj.x) + fabsf(ui.x) + fabsf(fx));
@@ -266,9 +273,14 @@ __device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { r
 // Pass A of component h of particle i (stretch tests, D, penalty sum, stress,
 // W).  All 32 lanes of the warp call it, lanes 2k and 2k + 1 with the same
 // particle; ok = false: the lane has none.
-// Bonds are taken kWalkA at a time: the group's bond data and its neighbours'
-// state are requested together, and the next group's indices with them, so a
-// group costs one memory latency.
+// Bonds are taken kWalkA at a time: while one group's terms are summed the next
+// one's bond data and neighbours' state are on their way, and the indices of the
+// one after it.  Without bond breaking a group has no branch (an empty slot's terms
+// are -0, which changes no sum).  In a plate too small to fill the chip a warp has
+// its SM quarter to itself and waits for each of these in turn (step, us, against
+// one group at a time: 30 x 31 particles 17.4 -> 13.6, with bonds breaking 16.5 ->
+// 14.1; 100 x 100 17.7 -> 14.4, 17.4 -> 15.8; 401 x 399 120.4 -> 113.9, 120.9 ->
+// 118.4; 1M 683 -> 664, 688 -> 684; 250 x 250 52.2 -> 50.1, but 51.7 -> 53.2).
 template <bool BREAK, bool HG>
 __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, int h, bool ok) {
   int w = 0;
@@ -283,53 +295,72 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   const FpConst K = fp_const(a);
   double d1 = 0.0, d2 = 0.0, ah = 0.0;  // row h of D, component h of the penalty sum
   int newly = 0;
-  const float s2 = BREAK ? (float)a.s2 : 0.f;
-  int jn[kWalkA];
-#pragma unroll
-  for (int q = 0; q < kWalkA; ++q) jn[q] = q < w ? a.nbr[s0 + (int64_t)q * kChunk] : -1;
-  for (int k = 0; k < w; k += kWalkA) {
-    const int64_t s = s0 + (int64_t)k * kChunk;
+  const float s2 = BREAK ? a.s2f : 0.f;
+  struct Group {
     int j[kWalkA];
     double uj[kWalkA], vj[kWalkA];
     double2 t[kWalkA];
     float2 uj32[kWalkA], e32[kWalkA];
+  };
+  int jn[kWalkA];
+  auto indices = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kWalkA; ++q) jn[q] = k + q < w ? a.nbr[s0 + (int64_t)(k + q) * kChunk] : -1;
+  };
+  auto request = [&](Group& g, int k) {
+    const int64_t s = s0 + (int64_t)k * kChunk;
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
-      j[q] = jn[q];
-      const int64_t jj = j[q] < 0 ? i : (int64_t)j[q];  // (an empty slot reads the particle itself)
-      const int64_t sq = j[q] < 0 ? s : s + (int64_t)q * kChunk;
-      uj[q] = comp(a.u, jj, h);
-      t[q] = __ldcs(&a.bgeo[sq]);
-      if (HG) vj[q] = a.vol[jj];
+      g.j[q] = jn[q];
+      const int64_t jj = g.j[q] < 0 ? i : (int64_t)g.j[q];  // (an empty slot reads the particle itself)
+      const int64_t sq = g.j[q] < 0 ? s0 : s + (int64_t)q * kChunk;
+      g.uj[q] = comp(a.u, jj, h);
+      g.t[q] = __ldcs(&a.bgeo[sq]);
+      if (HG) g.vj[q] = a.vol[jj];
       if (BREAK) {
-        uj32[q] = a.u32[jj];
-        e32[q] = __ldcs(&a.bxi32[sq]);
+        g.uj32[q] = a.u32[jj];
+        g.e32[q] = __ldcs(&a.bxi32[sq]);
       }
     }
-#pragma unroll
-    for (int q = 0; q < kWalkA; ++q)
-      jn[q] = k + kWalkA + q < w ? a.nbr[s + (int64_t)(kWalkA + q) * kChunk] : -1;
+  };
+  auto sums = [&](const Group& g, int k) {
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
-      if (j[q] < 0) continue;
+      const bool on = g.j[q] >= 0;
       if (BREAK) {
-        const int v = stretch_fp32(ui32, uj32[q], e32[q], s2);
-        if (v <= 0 && (v < 0 || stretch_fp64(a, i, j[q], s + (int64_t)q * kChunk))) {
+        if (!on) continue;
+        const int v = stretch_fp32(ui32, g.uj32[q], g.e32[q], s2);
+        const int64_t s = s0 + (int64_t)(k + q) * kChunk;
+        if (v <= 0 && (v < 0 || stretch_fp64(a, i, g.j[q], s))) {
           // both threads of the pair find the same; the second one does not store, and if it
           // reads the slot after the first one's store it skips the bond there
-          if (h == 0) a.nbr[s + (int64_t)q * kChunk] = -2 - j[q];
+          if (h == 0) a.nbr[s] = -2 - g.j[q];
           ++newly;
           continue;
         }
       }
-      const double dh = sub1(K, uj[q], ui);
-      d1 = fma(dh, t[q].x, d1);
-      d2 = fma(dh, t[q].y, d2);
-      if (HG) ah = fma(vj[q], dh, ah);
+      const double dh = BREAK || on ? sub1(K, g.uj[q], ui) : -0.0;
+      d1 = fma(dh, BREAK || on ? g.t[q].x : 1.0, d1);
+      d2 = fma(dh, BREAK || on ? g.t[q].y : 1.0, d2);
+      if (HG) ah = fma(BREAK || on ? g.vj[q] : 1.0, dh, ah);
+    }
+  };
+  if (w > 0) {
+    Group g0, g1;
+    indices(0);
+    request(g0, 0);
+    indices(kWalkA);
+    for (int k = 0; k < w; k += 2 * kWalkA) {
+      request(g1, k + kWalkA);
+      indices(k + 2 * kWalkA);
+      sums(g0, k);
+      request(g0, k + 2 * kWalkA);
+      indices(k + 3 * kWalkA);
+      if (k + kWalkA < w) sums(g1, k + kWalkA);
     }
   }
   // late, so that the next pass's blocks do not take the places of this pass's waiting ones
-  grid_dep_launch();
+  if (!a.exit_trigger) grid_dep_launch();
   if (HG && ok) set_comp(a.hg, i, h, mul1(K, a.k_hg2, ah));
   if (BREAK) {
     newly = __shfl_sync(0xffffffffu, newly, threadIdx.x & 30);  // the first thread's count
@@ -366,8 +397,10 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   (h ? a.w23 : a.w01)[i] = W;
 }
 
+// (10 blocks per SM, pass B 12: with registers to spare the compiler keeps the walk's
+// loads where they stand; left to itself it saves registers and moves them to their uses)
 template <bool BREAK, bool HG>
-__global__ void __launch_bounds__(kPairBlock) k_pass_a(Fp64Args a) {
+__global__ void __launch_bounds__(kPairBlock, 10) k_pass_a(Fp64Args a) {
   const int64_t i = a.i0 + (int64_t)blockIdx.x * (kPairBlock / 2) + (threadIdx.x >> 1);
   grid_dep_wait();  // nothing is read before the previous pass has completed
   pass_a_particle<BREAK, HG>(a, i, threadIdx.x & 1, i < a.n);
@@ -384,30 +417,47 @@ __device__ __forceinline__ void pass_b_particle(const Fp64Args& a, const FpConst
   double f = fma(wi.x, m.x, HG ? fma(wi.y, m.y, comp(a.hg, i, h)) : mul1(K, wi.y, m.y));
   // requested before the walk (1M-particle plate: 252 -> 243 us)
   double v = comp(a.v, i, h), ao = comp(MODE == 2 ? a.acc : a.f, i, h), u = MODE == 1 ? comp(a.u, i, h) : 0.0;
-  int jn[kWalkB];
-#pragma unroll
-  for (int q = 0; q < kWalkB; ++q) jn[q] = q < w ? __ldcs(&a.nbr[s0 + (int64_t)q * kChunk]) : -1;
-  for (int k = 0; k < w; k += kWalkB) {  // as pass A's walk
-    const int64_t s = s0 + (int64_t)k * kChunk;
+  struct Group {
     int j[kWalkB];
     double2 nb[kWalkB], e[kWalkB];
+  };
+  int jn[kWalkB];
+  auto indices = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kWalkB; ++q) jn[q] = k + q < w ? __ldcs(&a.nbr[s0 + (int64_t)(k + q) * kChunk]) : -1;
+  };
+  auto request = [&](Group& g, int k) {
+    const int64_t s = s0 + (int64_t)k * kChunk;
 #pragma unroll
     for (int q = 0; q < kWalkB; ++q) {
-      j[q] = jn[q];
-      nb[q] = W[j[q] < 0 ? i : (int64_t)j[q]];
-      e[q] = __ldcs(&a.bxi[j[q] < 0 ? s : s + (int64_t)q * kChunk]);
+      g.j[q] = jn[q];
+      g.nb[q] = W[g.j[q] < 0 ? i : (int64_t)g.j[q]];
+      g.e[q] = __ldcs(&a.bxi[g.j[q] < 0 ? s0 : s + (int64_t)q * kChunk]);
     }
-#pragma unroll
-    for (int q = 0; q < kWalkB; ++q)
-      jn[q] = k + kWalkB + q < w ? __ldcs(&a.nbr[s + (int64_t)(kWalkB + q) * kChunk]) : -1;
+  };
+  auto sums = [&](const Group& g) {
 #pragma unroll
     for (int q = 0; q < kWalkB; ++q) {
-      if (j[q] < 0) continue;
-      f = fma(nb[q].x, e[q].x, f);
-      f = fma(nb[q].y, e[q].y, f);
+      if (g.j[q] < 0) continue;
+      f = fma(g.nb[q].x, g.e[q].x, f);
+      f = fma(g.nb[q].y, g.e[q].y, f);
+    }
+  };
+  if (w > 0) {
+    Group g0, g1;
+    indices(0);
+    request(g0, 0);
+    indices(kWalkB);
+    for (int k = 0; k < w; k += 2 * kWalkB) {
+      request(g1, k + kWalkB);
+      indices(k + 2 * kWalkB);
+      sums(g0);
+      request(g0, k + 2 * kWalkB);
+      indices(k + 3 * kWalkB);
+      sums(g1);
     }
   }
-  grid_dep_launch();
+  if (!a.exit_trigger) grid_dep_launch();
   if (MODE != 2) ao = mul1(K, ao, a.inv_rho);
   const double an = mul1(K, f, a.inv_rho);
   v = add1(K, v, mul1(K, mul1(K, 0.5, add1(K, ao, an)), a.dt));
@@ -434,7 +484,7 @@ __device__ __forceinline__ void pass_b_particle(const Fp64Args& a, const FpConst
 }
 
 template <int MODE, bool HG>
-__global__ void __launch_bounds__(kPairBlock) k_pass_b(Fp64Args a) {
+__global__ void __launch_bounds__(kPairBlock, 12) k_pass_b(Fp64Args a) {
   const int64_t i = a.i0 + (int64_t)blockIdx.x * (kPairBlock / 2) + (threadIdx.x >> 1);
   grid_dep_wait();
   const FpConst K = fp_const(a);
@@ -577,7 +627,9 @@ static void launch_pass(void (*kernel)(Fp64Args), const Fp64Args& a, bool pdl, c
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = pdl ? 1 : 0;
-  cudaLaunchKernelEx(&lc, kernel, a);
+  Fp64Args b = a;
+  b.exit_trigger = a.n - a.i0 <= kExitTrigger;
+  cudaLaunchKernelEx(&lc, kernel, b);
 }
 
 void launch_pass_a_fp64(const Fp64Args& a, bool breaking, cudaStream_t s, bool pdl) {

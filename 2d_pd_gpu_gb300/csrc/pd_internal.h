@@ -104,7 +104,9 @@ struct Fp64Args {
   double one, neg_one, neg_zero;  // 1, -1, -0 (add1, sub1, mul1)
   double s2;                      // stretch limit factor (1 + s_c)^2 - 1 = s_c (2 + s_c)
   unsigned long long* counters;
-  int32_t brk;  // bond breaking on (s_c > 0)
+  float s2f;                      // s2 rounded to FP32 (converted in a walk, it would take the FP64 pipe per bond)
+  int32_t brk;                    // bond breaking on (s_c > 0)
+  int32_t exit_trigger;           // a pass lets the next one launch at its blocks' exit only (set at the launch)
   int32_t pad;
 };
 
