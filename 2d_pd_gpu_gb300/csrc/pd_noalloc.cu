@@ -28,6 +28,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "pd_internal.h"
 
@@ -117,6 +118,30 @@ __device__ __forceinline__ void store_a(const NoallocArgs& a, int64_t i, int h, 
 // for 64 cycles, so a thread's chain is what a call waits for.
 constexpr int kNoallocWalk = 4;  // bonds in flight per thread (2: 24.0 us against 21.6 per 30 x 31 call)
 
+// A warp's rows, up to `most` bonds: whole groups of bonds(k, their indices, the
+// group's size, what to request next), whose terms need no branch (a call on 256 x 255
+// particles 91.5 -> 90.2 us), then the rest one by one.
+template <typename Index, typename Bonds>
+__device__ __forceinline__ void walk_row(int64_t most, Index index, Bonds bonds) {
+  int jn[kNoallocWalk];
+  auto ask = [&](int64_t k) {
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) jn[q] = index(k + q);
+  };
+  int64_t k = 0;
+  ask(0);
+  for (; k + kNoallocWalk <= most; k += kNoallocWalk) {
+    int j[kNoallocWalk];
+#pragma unroll
+    for (int q = 0; q < kNoallocWalk; ++q) j[q] = jn[q];
+    bonds(k, j, std::integral_constant<int, kNoallocWalk>{}, [&] { ask(k + kNoallocWalk); });
+  }
+  for (; k < most; ++k) {
+    int j = index(k);
+    bonds(k, &j, std::integral_constant<int, 1>{}, [] {});
+  }
+}
+
 __global__ void __launch_bounds__(kNoallocBlock) k_noalloc_pass_a(NoallocArgs a) {
   const int64_t p = (int64_t)blockIdx.x * (kNoallocBlock / 2) + (threadIdx.x >> 1);
   const int h = threadIdx.x & 1;
@@ -130,43 +155,45 @@ __global__ void __launch_bounds__(kNoallocBlock) k_noalloc_pass_a(NoallocArgs a)
   const int64_t len = ok ? r1 - r0 : 0;
   const double one = in_register(a.one), neg1 = in_register(a.neg_one), neg0 = in_register(a.neg_zero);
   const int64_t most = longest(len);
-  int jn[kNoallocWalk];
-  auto ask = [&](int64_t k0) {
+  // the neighbour of bond k (past the row: the particle itself)
+  auto index = [&](int64_t k) { return k < len ? a.col[r0 + k] : (int)i; };
+  // U bonds j[0 .. U) from bond k on, without a branch each; next(): after their requests
+  auto bonds = [&](int64_t k, int* j, auto u, auto next) {
+    constexpr int U = decltype(u)::value;
+    double xj[U], uj[U], vj[U];
 #pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) jn[q] = k0 + q < len ? a.col[r0 + k0 + q] : (int)i;
-  };
-  ask(0);
-  for (int64_t k = 0; k < most; k += kNoallocWalk) {
-    double xj[kNoallocWalk], uj[kNoallocWalk], vj[kNoallocWalk];
-#pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) {
-      int j = jn[q];
-      if (j < 0 || j >= a.n) {  // a bad index: read nothing of it, poison this particle
+    for (int q = 0; q < U; ++q) {
+      if (j[q] < 0 || j[q] >= a.n) {  // a bad index: read nothing of it, poison this particle
         ok = false;
-        j = (int)i;
+        j[q] = (int)i;
       }
-      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j + h];
-      uj[q] = reinterpret_cast<const double*>(a.u)[2 * (int64_t)j + h];
-      vj[q] = a.vol[j];
+      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j[q] + h];
+      uj[q] = reinterpret_cast<const double*>(a.u)[2 * (int64_t)j[q] + h];
+      vj[q] = a.vol[j[q]];
     }
-    ask(k + kNoallocWalk);
+    next();
 #pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) {
-      const double e = fma(xi, neg1, xj[q]), t = fma(vj[q], e, neg0);
-      const double e2 = __shfl_xor_sync(0xffffffffu, e, 1), t2 = __shfl_xor_sync(0xffffffffu, t, 1);
-      if (k + q < len) {
-        const double tx = h ? t2 : t, ty = h ? t : t2;
-        ka = fma(t, e, ka);           // k11 | k22
-        if (h == 0) kb = fma(t, e2, kb);  // k12
-        m = fma(t, one, m);
-        const double d = fma(ui, neg1, uj[q]);
-        d1 = fma(d, tx, d1);
-        d2 = fma(d, ty, d2);
-        ah = fma(vj[q], d, ah);
+    for (int q = 0; q < U; ++q) {
+      double e = fma(xi, neg1, xj[q]), t = fma(vj[q], e, neg0), d = fma(ui, neg1, uj[q]);
+      if (k + q >= len) {  // zeros, which change no sum
+        e = t = 0.0;
+        d = -0.0;
+        vj[q] = 1.0;
       }
+      const double e2 = __shfl_xor_sync(0xffffffffu, e, 1), t2 = __shfl_xor_sync(0xffffffffu, t, 1);
+      const double tx = h ? t2 : t, ty = h ? t : t2;
+      ka = fma(t, e, ka);   // k11 | k22
+      kb = fma(t, e2, kb);  // k12 (h = 0)
+      m = fma(t, one, m);
+      d1 = fma(d, tx, d1);
+      d2 = fma(d, ty, d2);
+      ah = fma(vj[q], d, ah);
     }
-  }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  };
+  walk_row(most, index, bonds);
+  // (pass B is let go at the blocks' exit: launched while some SMs still hold blocks of this
+  // pass, its blocks crowd onto the others: calls on 120 x 120, 170 x 170 and 190 x 190 particles
+  // 29.8, 51.7 and 58.8 us against 24.6, 40.7 and 52.8)
   const double k11 = __shfl_sync(0xffffffffu, ka, threadIdx.x & 30), k12 = __shfl_sync(0xffffffffu, kb, threadIdx.x & 30),
                k22 = __shfl_sync(0xffffffffu, ka, (threadIdx.x & 30) + 1);
   const double det = fma(k11, k22, -(k12 * k12));
@@ -261,35 +288,30 @@ __global__ void __launch_bounds__(kNoallocBlock) k_noalloc_pass_b(NoallocArgs a)
   bool ok = row_ok(a, i, &r0, &r1);
   const int64_t len = ok ? r1 - r0 : 0, most = longest(len);
   const double neg1 = in_register(a.neg_one);
-  int jn[kNoallocWalk];
-  auto ask = [&](int64_t k0) {
+  auto index = [&](int64_t k) { return k < len ? a.col[r0 + k] : (int)i; };
+  auto bonds = [&](int64_t k, int* j, auto u, auto next) {
+    constexpr int U = decltype(u)::value;
+    double xj[U];
+    double2 wj[U];
 #pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) jn[q] = k0 + q < len ? a.col[r0 + k0 + q] : (int)i;
-  };
-  ask(0);
-  for (int64_t k = 0; k < most; k += kNoallocWalk) {
-    double xj[kNoallocWalk];
-    double2 wj[kNoallocWalk];
-#pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) {
-      int j = jn[q];
-      if (j < 0 || j >= a.n) {
+    for (int q = 0; q < U; ++q) {
+      if (j[q] < 0 || j[q] >= a.n) {
         ok = false;
-        j = (int)i;
+        j[q] = (int)i;
       }
-      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j + h];
-      wj[q] = Wr[j];
+      xj[q] = reinterpret_cast<const double*>(a.x)[2 * (int64_t)j[q] + h];
+      wj[q] = Wr[j[q]];
     }
-    ask(k + kNoallocWalk);
+    next();
 #pragma unroll
-    for (int q = 0; q < kNoallocWalk; ++q) {
+    for (int q = 0; q < U; ++q) {
       const double e = fma(xi, neg1, xj[q]), e2 = __shfl_xor_sync(0xffffffffu, e, 1);
-      if (k + q < len) {
-        f = fma(wj[q].x, h ? e2 : e, f);
-        f = fma(wj[q].y, h ? e : e2, f);
-      }
+      const bool on = k + q < len;  // past the row: -0, which changes no sum
+      f = fma(on ? wj[q].x : 1.0, on ? (h ? e2 : e) : -0.0, f);
+      f = fma(on ? wj[q].y : 1.0, on ? (h ? e : e2) : -0.0, f);
     }
-  }
+  };
+  walk_row(most, index, bonds);
   if (!ok) f = nan("");
   const double an = f * a.inv_rho;
   v = v + (0.5 * (ao + an)) * a.dt;

@@ -54,6 +54,13 @@ def test_noalloc_shapes_match_compute_velocity(pdg, nx, ny, horizon):
     ctx.close()
 
 
+@pytest.mark.parametrize("nx,ny,horizon", [(4097, 1, 1.015), (4111, 1, 2.015), (4099, 1, 3.015), (2051, 2, 1.015),
+                                           (2051, 2, 2.015), (1400, 3, 2.015), (1401, 3, 3.015), (90, 47, 3.5)])
+def test_noalloc_rows_past_whole_groups_match_compute_velocity(pdg, nx, ny, horizon):
+    """Rows of 1 to ~36 bonds: whole groups of four and 0 .. 3 bonds past them."""
+    test_noalloc_shapes_match_compute_velocity(pdg, nx, ny, horizon)
+
+
 @pytest.mark.parametrize("side", [40, 70])
 def test_noalloc_bad_index_poisons_its_particle(pdg, side):
     torch = pytest.importorskip("torch")
