@@ -38,7 +38,8 @@ __device__ __forceinline__ int64_t slot0(const Fp64Args& a, int64_t i, int* w) {
 constexpr int kPairBlock = 64;
 // Bonds per group of the passes' walks, two groups in flight (step with bonds
 // breaking, us, pass A 1, 2, 3 bonds: 100 x 100 particles 16.8, 16.3, 16.2, 1M 686,
-// 685, 711; pass B 2, 4: 1M 685, 710).
+// 685, 711; pass B 2, 4: 1M 685, 710).  With bond breaking each thread of a pair
+// runs the FP32 stretch test of one of a group's two bonds.
 constexpr int kWalkA = 2, kWalkB = 2;
 // Up to this many particles a pass lets the next one launch at its blocks' exit
 // only: launched while some SMs still hold blocks of this pass, the next one's
@@ -278,9 +279,9 @@ __device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { r
 // one after it.  Without bond breaking a group has no branch (an empty slot's terms
 // are -0, which changes no sum).  In a plate too small to fill the chip a warp has
 // its SM quarter to itself and waits for each of these in turn (step, us, against
-// one group at a time: 30 x 31 particles 17.4 -> 13.6, with bonds breaking 16.5 ->
-// 14.1; 100 x 100 17.7 -> 14.4, 17.4 -> 15.8; 401 x 399 120.4 -> 113.9, 120.9 ->
-// 118.4; 1M 683 -> 664, 688 -> 684; 250 x 250 52.2 -> 50.1, but 51.7 -> 53.2).
+// one group at a time: 30 x 31 particles 17.4 -> 13.5, with bonds breaking 16.5 ->
+// 13.7; 100 x 100 17.7 -> 14.5, 17.4 -> 15.5; 401 x 399 120.4 -> 113.9, 120.9 ->
+// 117.5; 1M 683 -> 664, 688 -> 683; 250 x 250 52.2 -> 49.8, but 51.7 -> 52.6).
 template <bool BREAK, bool HG>
 __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, int h, bool ok) {
   int w = 0;
@@ -300,8 +301,11 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
     int j[kWalkA];
     double uj[kWalkA], vj[kWalkA];
     double2 t[kWalkA];
-    float2 uj32[kWalkA], e32[kWalkA];
+    float2 uj32, e32;  // of the bond this thread tests
   };
+  static_assert(!BREAK || kWalkA == 2, "one bond of a group for each thread of the pair to test");
+  const int most = BREAK ? __reduce_max_sync(0xffffffffu, w) : w;  // (the pair exchanges run in every lane)
+  const int64_t self = BREAK && !ok ? a.n - 1 : i;                 // what an empty slot reads
   int jn[kWalkA];
   auto indices = [&](int k) {
 #pragma unroll
@@ -312,26 +316,32 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
       g.j[q] = jn[q];
-      const int64_t jj = g.j[q] < 0 ? i : (int64_t)g.j[q];  // (an empty slot reads the particle itself)
+      const int64_t jj = g.j[q] < 0 ? self : (int64_t)g.j[q];
       const int64_t sq = g.j[q] < 0 ? s0 : s + (int64_t)q * kChunk;
       g.uj[q] = comp(a.u, jj, h);
       g.t[q] = __ldcs(&a.bgeo[sq]);
       if (HG) g.vj[q] = a.vol[jj];
-      if (BREAK) {
-        g.uj32[q] = a.u32[jj];
-        g.e32[q] = __ldcs(&a.bxi32[sq]);
-      }
+    }
+    if (BREAK) {
+      const int jo = h ? g.j[1] : g.j[0];
+      g.uj32 = a.u32[jo < 0 ? self : (int64_t)jo];
+      g.e32 = __ldcs(&a.bxi32[jo < 0 ? s0 : s + (int64_t)h * kChunk]);
     }
   };
   auto sums = [&](const Group& g, int k) {
+    int v[2] = {1, 1};
+    if (BREAK) {  // (both bonds tested by both threads: 100 x 100 particles 16.0 against 15.5 us per step)
+      const int mine = stretch_fp32(ui32, g.uj32, g.e32, s2), other = __shfl_xor_sync(0xffffffffu, mine, 1);
+      v[0] = h ? other : mine;
+      v[1] = h ? mine : other;
+    }
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
       const bool on = g.j[q] >= 0;
       if (BREAK) {
         if (!on) continue;
-        const int v = stretch_fp32(ui32, g.uj32[q], g.e32[q], s2);
         const int64_t s = s0 + (int64_t)(k + q) * kChunk;
-        if (v <= 0 && (v < 0 || stretch_fp64(a, i, g.j[q], s))) {
+        if (v[q] <= 0 && (v[q] < 0 || stretch_fp64(a, i, g.j[q], s))) {
           // both threads of the pair find the same; the second one does not store, and if it
           // reads the slot after the first one's store it skips the bond there
           if (h == 0) a.nbr[s] = -2 - g.j[q];
@@ -345,18 +355,18 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
       if (HG) ah = fma(BREAK || on ? g.vj[q] : 1.0, dh, ah);
     }
   };
-  if (w > 0) {
+  if (most > 0) {
     Group g0, g1;
     indices(0);
     request(g0, 0);
     indices(kWalkA);
-    for (int k = 0; k < w; k += 2 * kWalkA) {
+    for (int k = 0; k < most; k += 2 * kWalkA) {
       request(g1, k + kWalkA);
       indices(k + 2 * kWalkA);
       sums(g0, k);
       request(g0, k + 2 * kWalkA);
       indices(k + 3 * kWalkA);
-      if (k + kWalkA < w) sums(g1, k + kWalkA);
+      if (k + kWalkA < most) sums(g1, k + kWalkA);
     }
   }
   // late, so that the next pass's blocks do not take the places of this pass's waiting ones
