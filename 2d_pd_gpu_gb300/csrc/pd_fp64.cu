@@ -61,8 +61,9 @@ __device__ __forceinline__ void set_comp(double2* p, int64_t i, int h, double v)
   reinterpret_cast<double*>(p)[2 * i + h] = v;
 }
 
-// K^-1 and m/V of particle i over its intact bonds (oracle: kinv_of).
-__device__ void kinv_update(const Fp64Args& a, int64_t i) {
+// K^-1 and m/V of particle i over its intact bonds (oracle: kinv_of); true: singular
+// (the caller counts it).
+__device__ bool kinv_update(const Fp64Args& a, int64_t i) {
   int w;
   const int64_t s0 = slot0(a, i, &w);
   double k11 = 0.0, k12 = 0.0, k22 = 0.0, mx = 0.0, my = 0.0;
@@ -87,8 +88,7 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
     a.kinv22[i] = 0.0;
     a.mt[i] = make_double2(0.0, 0.0);
     a.singular[i] = 1;
-    atomicAdd(a.counters + CNT_SINGULAR, 1ull);
-    return;
+    return true;
   }
   const double r = 1.0 / det;
   a.kinv01[i] = make_double2(k22 * r, -k12 * r);
@@ -96,7 +96,14 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
   const double rv = 1.0 / a.vol[i];
   a.mt[i] = make_double2(mx * rv, my * rv);
   a.singular[i] = 0;
+  return false;
 }
+
+// From more than this many of a warp's particles on, each updates itself: the warp
+// form takes ~19 FP64 instructions of the pipe per particle, one lane each ~180 in all
+// (a step in which all of 1M particles lose bonds 1902 -> 1127 us, of which the counters'
+// one addition per warp instead of per particle is most).
+constexpr int kManyLost = 8;
 
 // Pass A's update of the particles that lost bonds (newly > 0 in their lane):
 // broken count, damage, K^-1 and m/V, by the whole warp.  Eight lanes take a
@@ -110,6 +117,21 @@ __device__ void kinv_update(const Fp64Args& a, int64_t i) {
 __device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int64_t s0, int w, int newly) {
   const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
   unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
+  if (__popc(todo) > kManyLost) {
+    bool bad = false;
+    if (newly > 0) {
+      const int32_t broken = a.broken[i] + newly;
+      a.broken[i] = broken;
+      a.damage[i] = (double)broken / (double)a.fam[i];
+      bad = kinv_update(a, i);
+    }
+    const int all = __reduce_add_sync(0xffffffffu, newly), nbad = __popc(__ballot_sync(0xffffffffu, bad));
+    if (lane == 0) {
+      atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)all);
+      if (nbad) atomicAdd(a.counters + CNT_SINGULAR, (unsigned long long)nbad);
+    }
+    return;
+  }
   while (todo) {
     unsigned rest = todo;  // this lane's particle: that of the (lane / 8)-th lane left to do
     for (int q = lane >> 3; q > 0; --q) rest &= rest - 1;
@@ -177,8 +199,7 @@ __device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int6
 
 __global__ void __launch_bounds__(kBlock) k_init_geometry(Fp64Args a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  kinv_update(a, i);
+  if (i < a.n && kinv_update(a, i)) atomicAdd(a.counters + CNT_SINGULAR, 1ull);
 }
 
 // Velocity BC, drift, fixed BC of particle i; an = f_i / rho.

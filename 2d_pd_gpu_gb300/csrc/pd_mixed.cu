@@ -73,8 +73,9 @@ __device__ __forceinline__ void split2(double v, float& hi, float& lo) {
 }
 
 // K^-1 (FP64 inversion + guard) and m^ from the FP64 reference positions of
-// particle i at SELL position p, whose slots are s0 + 32 k, k < w.
-__device__ void kinv_update_mixed(const MixedArgs& a, int64_t i, int64_t p, int64_t s0, int w) {
+// particle i at SELL position p, whose slots are s0 + 32 k, k < w; true: singular (the
+// caller counts it).
+__device__ bool kinv_update_mixed(const MixedArgs& a, int64_t i, int64_t p, int64_t s0, int w) {
   const double2 xi = a.x[i];
   double k11 = 0.0, k12 = 0.0, k22 = 0.0, mx = 0.0, my = 0.0;
   int nal = 0;
@@ -101,13 +102,13 @@ __device__ void kinv_update_mixed(const MixedArgs& a, int64_t i, int64_t p, int6
     a.geo[p] = make_float4(0.f, 0.f, 0.f, (float)vi);
     a.mh[p] = make_float2(0.f, 0.f);
     a.singular[p] = 1;
-    atomicAdd(a.counters + CNT_SINGULAR, 1ull);
-    return;
+    return true;
   }
   const double r = 1.0 / det;
   a.geo[p] = make_float4((float)(k22 * r), (float)(-k12 * r), (float)(k11 * r), (float)vi);
   a.mh[p] = make_float2((float)(mx / vi), (float)(my / vi));
   a.singular[p] = 0;
+  return false;
 }
 
 // W^ = V^ (sigma^ K^-1 - k^ G) of a particle from its D (D1 = (d11, d12), D2 =
@@ -126,6 +127,12 @@ __device__ __forceinline__ float4 w_of(const MixedArgs& a, float2 D1, float2 D2,
                      vi * fmaf(kh, g12, fmaf(s11, k12, s12 * k22)), vi * fmaf(kh, g22, fmaf(s12, k12, s22 * k22)));
 }
 
+// From more than this many of a warp's particles on, each updates itself: the warp
+// form takes ~21 FP64 instructions of the pipe per particle, one lane each ~300 in all
+// (a step in which all of 1M particles lose bonds 1510 -> 805 us, of which the counters'
+// one addition per warp instead of per particle is most; 160,000 particles 424 -> 184).
+constexpr int kManyLost = 14;
+
 // Pass A's update of the particles that lost bonds (newly > 0 in their lane, p
 // its SELL position, s0 and w its slots): broken count, damage, K^-1, m^ and W^, by the whole warp;
 // D: the lanes' sums in shared memory (the call has few registers to save then).
@@ -140,6 +147,24 @@ __device__ __noinline__ void kinv_update_mixed_warp(const MixedArgs& a, int64_t 
   constexpr int kPer = 4;  // bonds per lane and round
   const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
   unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
+  if (__popc(todo) > kManyLost) {
+    bool bad = false;
+    if (newly > 0) {
+      const int64_t i = a.member[p];
+      const int32_t broken = a.broken[i] + newly;
+      a.broken[i] = broken;
+      a.damage[i] = (double)broken / (double)a.fam[i];
+      bad = kinv_update_mixed(a, i, p, s0, w);
+      const float4 d = D[lane];
+      a.ws[p] = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, f2(d.x, d.y), f2(d.z, d.w), a.geo[p]);
+    }
+    const int all = __reduce_add_sync(0xffffffffu, newly), nbad = __popc(__ballot_sync(0xffffffffu, bad));
+    if (lane == 0) {
+      atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)all);
+      if (nbad) atomicAdd(a.counters + CNT_SINGULAR, (unsigned long long)nbad);
+    }
+    return;
+  }
   while (todo) {
     unsigned rest = todo;  // this lane's particle: that of the (lane / 8)-th lane left to do
     for (int q = lane >> 3; q > 0; --q) rest &= rest - 1;
@@ -219,7 +244,7 @@ __global__ void __launch_bounds__(kBlock) k_init_geometry_mixed(MixedArgs a) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const int64_t p = sell_pos(a.pos_of, i);
-  kinv_update_mixed(a, i, p, sell_slot0(a.chunk_base, p), a.chunk_w[p >> 5]);
+  if (kinv_update_mixed(a, i, p, sell_slot0(a.chunk_base, p), a.chunk_w[p >> 5])) atomicAdd(a.counters + CNT_SINGULAR, 1ull);
 }
 
 // BC + drift of particle i in scaled per-step units; an = a^ of the new force.
