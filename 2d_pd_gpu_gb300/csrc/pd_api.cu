@@ -323,11 +323,15 @@ int ensure_ba(pd_ctx* c) {
   if (!c->ba_kq0) PD_CK(c, cudaMalloc(&c->ba_kq0, ns * sizeof(double2)));
   if (!c->ba_kq1) PD_CK(c, cudaMalloc(&c->ba_kq1, ns * sizeof(double2)));
   if (!c->ba_rv) PD_CK(c, cudaMalloc(&c->ba_rv, (size_t)(c->n > 0 ? c->n : 1) * sizeof(double)));
-  if (!c->ba_wfull)
-    PD_CK(c, cudaMalloc(&c->ba_wfull, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaFull * sizeof(double)));
-  pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
   if (!c->rslot) PD_CK(c, cudaMalloc(&c->rslot, ns * sizeof(int64_t)));
   PD_CK(c, cudaMalloc(&c->tb, ns * sizeof(double2)));
+  // (8 KB per particle: where it does not fit, the passes evaluate the weights; the same results)
+  if (!c->ba_wfull &&
+      cudaMalloc(&c->ba_wfull, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaFull * sizeof(double)) != cudaSuccess) {
+    c->ba_wfull = nullptr;
+    cudaGetLastError();
+  }
+  pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
   PD_CK(c, cudaMemsetAsync(c->tb, 0, ns * sizeof(double2), c->stream));
   PD_CK(c, cudaMemsetAsync(c->counters + pd::CNT_ERROR, 0, sizeof(unsigned long long), c->stream));
   pd::launch_ba_reverse(fp64_args(c), ba_args(c), c->stream);

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
   for (int o = 16; o; o >>= 1) lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
   wf.direct = !(fabs(b.n1) * lmax * b.inv_wlen < 600.0);
   __syncwarp();
-  const bool tri = n <= 32;
+  const bool tri = n <= 32 && b.wfull != nullptr;
   if (tri) {
     double* wt = b.wfull + i * kBaFull;
     if (KTAB) {  // pair p = k (k + 1) / 2 + q, q <= k, of the lower triangle, evaluated and kept
@@ -486,7 +486,7 @@ void launch_ba_bonds(const Fp64Args& a, const BondAssoc& b, int64_t nslots, cuda
 void launch_ba_pass_a(const Fp64Args& a, const BondAssoc& b, cudaStream_t s) {
   if (a.n <= 0) return;
   const unsigned nb = (unsigned)((a.n + kBaWarps - 1) / kBaWarps);
-  if (b.max_family <= 32)
+  if (b.max_family <= 32 && b.wfull)
     k_ba_pass_a_small<<<nb, 32 * kBaWarps, 0, s>>>(a, b);
   else
     k_ba_pass_a<false><<<nb, 32 * kBaWarps, 0, s>>>(a, b);

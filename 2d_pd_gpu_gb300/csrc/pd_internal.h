@@ -119,7 +119,7 @@ struct BondAssoc {
   double2* ex;     // per bond slot: exp(n1 |xi| / l), exp(-n1 |xi| / l) (for the weights n1, l of the call)
   double2* kq0;    // per bond slot: K_b^-1 (q11, q12)
   double2* kq1;    // per bond slot: (q22, 1 if K_b fails the det guard else 0)
-  double* wfull;   // per particle with <= 32 bonds: its weight matrix, w(q, k) at [k][q] (kBaFull doubles)
+  double* wfull;   // per particle with <= 32 bonds: its weight matrix, w(q, k) at [k][q] (kBaFull doubles); or null
   double* rv;      // per particle: 1 / its family's volume
   int32_t max_family, pad;
 };
