@@ -263,7 +263,7 @@ void stiffness(const pd_ctx* c, double* c11, double* c12, double* c33);
 
 Fp64Args fp64_args(pd_ctx* c) {
   Fp64Args a{};
-  a.n = c->n;
+  a.n = a.plate = c->n;
   a.x = c->x; a.vol = c->vol; a.u = c->u; a.v = c->v; a.f = c->f; a.acc = c->acc;
   a.w01 = c->w01; a.w23 = c->w23; a.kinv01 = c->kinv01; a.kinv22 = c->kinv22; a.mt = c->mt; a.hg = c->hg;
   a.bc = c->bc; a.gkind = c->gkind; a.gval = c->gval;

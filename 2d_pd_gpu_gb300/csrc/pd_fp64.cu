@@ -292,6 +292,53 @@ __device__ __forceinline__ double add1(const FpConst& a, double x, double y) { r
 __device__ __forceinline__ double sub1(const FpConst& a, double x, double y) { return fma(y, a.neg_one, x); }
 __device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { return fma(x, y, a.neg_zero); }
 
+// Pass A's stretch tests of particle i ahead of its sums, its bonds dealt to the two threads of
+// the pair in turn; broken ones are marked.  Returns the number this thread broke.
+constexpr int kTests = 7;  // in flight (1M particles: 2, 4, 7, 14: 712, 696, 684, 682 us per step at 10 blocks per SM)
+__device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, int64_t s0, int w, float2 ui32) {
+  int newly = 0, jn[kTests];
+  auto indices = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kTests; ++q) jn[q] = k + 2 * q < w ? a.nbr[s0 + (int64_t)(k + 2 * q) * kChunk] : -1;
+  };
+  indices(h);
+  for (int k = h; k < w; k += 2 * kTests) {
+    int j[kTests], least = 1;
+    float2 u[kTests], e[kTests];
+#pragma unroll
+    for (int q = 0; q < kTests; ++q) {
+      j[q] = jn[q];
+      u[q] = a.u32[j[q] < 0 ? i : (int64_t)j[q]];
+      e[q] = __ldcs(&a.bxi32[j[q] < 0 ? s0 : s0 + (int64_t)(k + 2 * q) * kChunk]);
+    }
+    indices(k + 2 * kTests);
+    int v[kTests];
+#pragma unroll
+    for (int q = 0; q < kTests; ++q) {
+      v[q] = j[q] >= 0 ? stretch_fp32(ui32, u[q], e[q], a.s2f) : 1;
+      least = min(least, v[q]);
+    }
+    if (least <= 0) {
+#pragma unroll
+      for (int q = 0; q < kTests; ++q) {
+        const int64_t s = s0 + (int64_t)(k + 2 * q) * kChunk;
+        if (v[q] <= 0 && (v[q] < 0 || stretch_fp64(a, i, j[q], s))) {
+          a.nbr[s] = -2 - j[q];
+          ++newly;
+        }
+      }
+    }
+  }
+  return newly;
+}
+
+// From this many particles (of the plate) on, pass A tests a particle's bonds before it sums them:
+// the sums then need 72 registers instead of 96 and no branch, and other warps' sums keep the FP64
+// pipe busy under the tests (step with bonds breaking, us, 500 x 500 particles 176.7 -> 175.9,
+// 800 x 800 441 -> 435, 1M 683.5 -> 672, 2M 1356 -> 1329).  A smaller plate waits for the tests
+// (400 x 400 117.5 -> 118.1, 100 x 100 15.3 -> 15.9).
+constexpr int64_t kTestsFirst = 250000;
+
 // Pass A of component h of particle i (stretch tests, D, penalty sum, stress,
 // W).  All 32 lanes of the warp call it, lanes 2k and 2k + 1 with the same
 // particle; ok = false: the lane has none.
@@ -303,7 +350,7 @@ __device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { r
 // one group at a time: 30 x 31 particles 17.4 -> 13.5, with bonds breaking 16.5 ->
 // 13.7; 100 x 100 17.7 -> 14.5, 17.4 -> 15.5; 401 x 399 120.4 -> 113.9, 120.9 ->
 // 117.5; 1M 683 -> 664, 688 -> 683; 250 x 250 52.2 -> 49.8, but 51.7 -> 52.6).
-template <bool BREAK, bool HG>
+template <bool BREAK, bool HG, bool TESTS_FIRST>
 __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, int h, bool ok) {
   int w = 0;
   int64_t s0 = 0;
@@ -317,16 +364,22 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   const FpConst K = fp_const(a);
   double d1 = 0.0, d2 = 0.0, ah = 0.0;  // row h of D, component h of the penalty sum
   int newly = 0;
-  const float s2 = BREAK ? a.s2f : 0.f;
+  constexpr bool TEST = BREAK && !TESTS_FIRST;  // among the sums
+  if (BREAK && TESTS_FIRST) {
+    newly = test_bonds(a, i, h, s0, w, ui32);
+    newly += __shfl_xor_sync(0xffffffffu, newly, 1);
+    __syncwarp();  // (the marks are read by both threads)
+  }
+  const float s2 = TEST ? a.s2f : 0.f;
   struct Group {
     int j[kWalkA];
     double uj[kWalkA], vj[kWalkA];
     double2 t[kWalkA];
     float2 uj32, e32;  // of the bond this thread tests
   };
-  static_assert(!BREAK || kWalkA == 2, "one bond of a group for each thread of the pair to test");
-  const int most = BREAK ? __reduce_max_sync(0xffffffffu, w) : w;  // (the pair exchanges run in every lane)
-  const int64_t self = BREAK && !ok ? a.n - 1 : i;                 // what an empty slot reads
+  static_assert(!TEST || kWalkA == 2, "one bond of a group for each thread of the pair to test");
+  const int most = TEST ? __reduce_max_sync(0xffffffffu, w) : w;  // (the pair exchanges run in every lane)
+  const int64_t self = TEST && !ok ? a.n - 1 : i;                 // what an empty slot reads
   int jn[kWalkA];
   auto indices = [&](int k) {
 #pragma unroll
@@ -343,7 +396,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
       g.t[q] = __ldcs(&a.bgeo[sq]);
       if (HG) g.vj[q] = a.vol[jj];
     }
-    if (BREAK) {
+    if (TEST) {
       const int jo = h ? g.j[1] : g.j[0];
       g.uj32 = a.u32[jo < 0 ? self : (int64_t)jo];
       g.e32 = __ldcs(&a.bxi32[jo < 0 ? s0 : s + (int64_t)h * kChunk]);
@@ -351,7 +404,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   };
   auto sums = [&](const Group& g, int k) {
     int v[2] = {1, 1};
-    if (BREAK) {  // (both bonds tested by both threads: 100 x 100 particles 16.0 against 15.5 us per step)
+    if (TEST) {  // (both bonds tested by both threads: 100 x 100 particles 16.0 against 15.5 us per step)
       const int mine = stretch_fp32(ui32, g.uj32, g.e32, s2), other = __shfl_xor_sync(0xffffffffu, mine, 1);
       v[0] = h ? other : mine;
       v[1] = h ? mine : other;
@@ -359,7 +412,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
 #pragma unroll
     for (int q = 0; q < kWalkA; ++q) {
       const bool on = g.j[q] >= 0;
-      if (BREAK) {
+      if (TEST) {
         if (!on) continue;
         const int64_t s = s0 + (int64_t)(k + q) * kChunk;
         if (v[q] <= 0 && (v[q] < 0 || stretch_fp64(a, i, g.j[q], s))) {
@@ -370,10 +423,10 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
           continue;
         }
       }
-      const double dh = BREAK || on ? sub1(K, g.uj[q], ui) : -0.0;
-      d1 = fma(dh, BREAK || on ? g.t[q].x : 1.0, d1);
-      d2 = fma(dh, BREAK || on ? g.t[q].y : 1.0, d2);
-      if (HG) ah = fma(BREAK || on ? g.vj[q] : 1.0, dh, ah);
+      const double dh = TEST || on ? sub1(K, g.uj[q], ui) : -0.0;
+      d1 = fma(dh, TEST || on ? g.t[q].x : 1.0, d1);
+      d2 = fma(dh, TEST || on ? g.t[q].y : 1.0, d2);
+      if (HG) ah = fma(TEST || on ? g.vj[q] : 1.0, dh, ah);
     }
   };
   if (most > 0) {
@@ -394,7 +447,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   if (!a.exit_trigger) grid_dep_launch();
   if (HG && ok) set_comp(a.hg, i, h, mul1(K, a.k_hg2, ah));
   if (BREAK) {
-    newly = __shfl_sync(0xffffffffu, newly, threadIdx.x & 30);  // the first thread's count
+    if (TEST) newly = __shfl_sync(0xffffffffu, newly, threadIdx.x & 30);  // the first thread's count
     if (__any_sync(0xffffffffu, newly != 0)) kinv_update_warp(a, i, s0, w, h == 0 ? newly : 0);
   }
   double2 k01 = make_double2(0.0, 0.0);
@@ -430,11 +483,11 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
 
 // (10 blocks per SM, pass B 12: with registers to spare the compiler keeps the walk's
 // loads where they stand; left to itself it saves registers and moves them to their uses)
-template <bool BREAK, bool HG>
-__global__ void __launch_bounds__(kPairBlock, 10) k_pass_a(Fp64Args a) {
+template <bool BREAK, bool HG, bool TESTS_FIRST = false>
+__global__ void __launch_bounds__(kPairBlock, TESTS_FIRST ? 12 : 10) k_pass_a(Fp64Args a) {
   const int64_t i = a.i0 + (int64_t)blockIdx.x * (kPairBlock / 2) + (threadIdx.x >> 1);
   grid_dep_wait();  // nothing is read before the previous pass has completed
-  pass_a_particle<BREAK, HG>(a, i, threadIdx.x & 1, i < a.n);
+  pass_a_particle<BREAK, HG, TESTS_FIRST>(a, i, threadIdx.x & 1, i < a.n);
 }
 
 // Pass B of component h of particle i (force gather, kick; MODE 1 adds the
@@ -530,9 +583,9 @@ __device__ __forceinline__ void batch_particle(const Fp64Args& p, int64_t i, int
     if (ok && h == 0) drift_particle(p, i);
   } else if (phase == 1) {
     if (p.brk)
-      hg ? pass_a_particle<true, true>(p, i, h, ok) : pass_a_particle<true, false>(p, i, h, ok);
+      hg ? pass_a_particle<true, true, false>(p, i, h, ok) : pass_a_particle<true, false, false>(p, i, h, ok);
     else
-      hg ? pass_a_particle<false, true>(p, i, h, ok) : pass_a_particle<false, false>(p, i, h, ok);
+      hg ? pass_a_particle<false, true, false>(p, i, h, ok) : pass_a_particle<false, false, false>(p, i, h, ok);
   } else {
     const FpConst K = fp_const(p);
     if (!ok) return;
@@ -666,7 +719,9 @@ static void launch_pass(void (*kernel)(Fp64Args), const Fp64Args& a, bool pdl, c
 void launch_pass_a_fp64(const Fp64Args& a, bool breaking, cudaStream_t s, bool pdl) {
   if (a.n <= a.i0) return;
   const bool hg = a.k_hg != 0.0;
-  if (breaking)
+  if (breaking && a.plate >= kTestsFirst)
+    launch_pass(hg ? k_pass_a<true, true, true> : k_pass_a<true, false, true>, a, pdl, s);
+  else if (breaking)
     launch_pass(hg ? k_pass_a<true, true> : k_pass_a<true, false>, a, pdl, s);
   else
     launch_pass(hg ? k_pass_a<false, true> : k_pass_a<false, false>, a, pdl, s);

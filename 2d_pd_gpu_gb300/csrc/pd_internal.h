@@ -60,6 +60,7 @@ enum { ERR_FAMILY_OVERFLOW = 1, ERR_BAD_NEIGHBOR = 2, ERR_SELF_BOND = 4, ERR_ASY
 struct Fp64Args {
   int64_t n;
   int64_t i0;  // drift and the passes run particles i0 <= i < n (a slab; 0 for the whole plate)
+  int64_t plate;  // particles of the whole plate
   const double2* __restrict__ x;
   const double* __restrict__ vol;
   double2* u;

@@ -43,3 +43,11 @@ def test_every_walk_width_matches_oracle(pdg, po, shape, penalty, s_c):
 def test_hand_over_by_size_matches_oracle(pdg, po, shape, s_c):
     p = pdg.plates.make_plate(shape[0], shape[1], seed=12, crack="centre-half")
     _compare(pdg, po, p, s_c, p.k_hg, 4)
+
+
+@pytest.mark.parametrize("penalty", [False, True])
+@pytest.mark.parametrize("shape", [(125001, 2), (62501, 4), (501, 500)])
+def test_tests_ahead_of_the_sums_match_oracle(pdg, po, shape, penalty):
+    """From 250,000 particles on, bonds are tested before a particle's sums: narrow and wide chunks."""
+    p = pdg.plates.make_plate(shape[0], shape[1], seed=13)
+    _compare(pdg, po, p, 5e-4, p.k_hg if penalty else 0.0, 2)

@@ -2,7 +2,8 @@
 state equal the oracle's bit for bit where the FP32 stretch test cannot decide
 (stretches within rounding of s_c), where it decides either way, and under a
 rigid translation that is large against the bonds' elongations; with one, some
-and all of a warp's particles (16 per warp) losing bonds in a step."""
+and all of a warp's particles (16 per warp) losing bonds in a step; and either
+side of 250,000 particles, from where on the tests run ahead of the sums."""
 import numpy as np
 import pytest
 
@@ -35,3 +36,9 @@ def test_bonds_at_the_critical_stretch_match_oracle(pdg, po, shape, rel, shift):
     assert np.array_equal(gu, sim.u) and np.array_equal(gv, sim.v) and np.array_equal(gf, sim.f)
     assert ctx.counters()["bonds_broken"] == int((sim.mask == 0).sum())
     ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(499, 501), (500, 500)])
+@pytest.mark.parametrize("rel", [-1e-12, 0.0, 5e-7, 1e-2])
+def test_tests_ahead_of_the_sums_match_oracle(pdg, po, shape, rel):
+    test_bonds_at_the_critical_stretch_match_oracle(pdg, po, shape, rel, 3e-2)
