@@ -174,7 +174,7 @@ def byte_model(precision, n, nb):
 # and profiles/passes_mixed_plate600.txt), scaled to a launch by its bonds:
 # traffic grows with the bonds (and the particles, in the same proportion on
 # these plates).
-DRAM_BYTES_PER_BOND = {"fp64": {"pass_a": 308.52e6 / 10031592, "pass_b": 246.79e6 / 10031592},
+DRAM_BYTES_PER_BOND = {"fp64": {"pass_a": 308.19e6 / 10031592, "pass_b": 246.97e6 / 10031592},
                        "mixed": {"pass_a": 41.69e6 / 10031592, "pass_b": 55.45e6 / 10031592}}
 
 
