@@ -448,7 +448,10 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   if (HG && ok) set_comp(a.hg, i, h, mul1(K, a.k_hg2, ah));
   if (BREAK) {
     if (TEST) newly = __shfl_sync(0xffffffffu, newly, threadIdx.x & 30);  // the first thread's count
-    if (__any_sync(0xffffffffu, newly != 0)) kinv_update_warp(a, i, s0, w, h == 0 ? newly : 0);
+    if (__any_sync(0xffffffffu, newly != 0)) {
+      __syncwarp();  // (other lanes read the marks)
+      kinv_update_warp(a, i, s0, w, h == 0 ? newly : 0);
+    }
   }
   double2 k01 = make_double2(0.0, 0.0);
   double k22 = 0.0, vi = 0.0;
