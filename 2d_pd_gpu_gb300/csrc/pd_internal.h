@@ -198,6 +198,7 @@ struct MixedArgs {
   double2* out_v;
   double2* out_f;
   int64_t blk0;
+  int32_t exit_trigger;  // a pass lets the next one launch at its blocks' exit only (set at the launch)
   int32_t uniform_v;  // every particle's V^ is exactly 1 (pass A leaves the V^ gathers out)
 };
 

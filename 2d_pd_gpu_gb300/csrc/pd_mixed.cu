@@ -607,7 +607,7 @@ __device__ __forceinline__ void for_halo(const int32_t* H, int hn, int (&g)[kHal
 // Pass A of visiting block blk (kHaloBlock / 32 chunks) of plate a.  Every
 // thread of the kHaloBlock-thread block calls it; sm = the pass's dynamic
 // shared memory.  False if a staged copy timed out.  PDL: the pass may start
-// before the previous one has finished; until grid_dep_sync() it reads only
+// before the previous one has finished; until grid_dep_wait() it reads only
 // the visit record and the first halo ids, which no step writes.
 template <bool BREAK, bool PDL = false, bool UV = false>
 __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, unsigned char* sm, uint64_t* bars) {
@@ -621,7 +621,8 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
   int g[kHaloBatch];
   if (PDL) {
     if (hn >= 0) halo_ids(a.halo + blk * a.halo_cap, hn, 0, g);
-    grid_dep_sync();
+    grid_dep_wait();
+    if (!a.exit_trigger) grid_dep_launch();
   }
   PreA pre{};
   if (live) pre = load_a(a, p);  // in flight during the staging below
@@ -671,7 +672,8 @@ __device__ __forceinline__ bool pass_b_block(const MixedArgs& a, int64_t blk, un
   int g[kHaloBatch];
   if (PDL) {
     if (hn >= 0) halo_ids(a.halo + blk * a.halo_cap, hn, 0, g);
-    grid_dep_sync();
+    grid_dep_wait();
+    if (!a.exit_trigger) grid_dep_launch();
   }
   PreB pre{};
   if (live) pre = load_b<DRIFT, EXPORT>(a, p);  // in flight during the staging below
@@ -1225,6 +1227,14 @@ static void (*pass_a_kernel(const MixedArgs& a, bool breaking))(MixedArgs) {
   return breaking ? k_pass_a_mixed<true, false> : k_pass_a_mixed<false, false>;
 }
 
+// Passes of more than two and up to three blocks per SM (four fit) let the next one launch at
+// their blocks' exit only: launched at their start, its blocks fill the fourth places and then those
+// of the blocks that end first, and some SMs run more of them than others (step, us, without / with
+// bonds breaking: 280 x 280 particles 13.5 -> 11.4 / 14.9 -> 12.9, 320 x 320 13.9 -> 12.0 / 16.6 ->
+// 14.7).  Up to two per SM both passes' blocks have their places at once (260 x 260 8.7 us; at the
+// exit 9.4), and a longer pass evens itself out (1M 82 us; 83.6).
+constexpr int64_t kExitFrom = 2 * 152, kExitTo = 3 * 152;
+
 static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_t sm, cudaStream_t s,
                             bool pdl = true) {
   if (a.nblocks <= a.blk0) return;
@@ -1238,7 +1248,9 @@ static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = pdl ? 1 : 0;
-  cudaLaunchKernelEx(&lc, kernel, a);
+  MixedArgs b = a;
+  b.exit_trigger = a.nblocks - a.blk0 > kExitFrom && a.nblocks - a.blk0 <= kExitTo;
+  cudaLaunchKernelEx(&lc, kernel, b);
 }
 
 void launch_pass_a_mixed(const MixedArgs& a, bool breaking, cudaStream_t s) {

@@ -20,15 +20,12 @@
 namespace pd {
 
 // Programmatic dependent launch: a pass launched with programmatic stream
-// serialization starts while the previous pass drains; grid_dep_sync() waits
-// until that pass has completed and its writes are visible, then lets the next
-// pass launch.  Without the launch attribute both instructions return at once.
+// serialization starts while the previous pass drains; grid_dep_wait() waits
+// until that pass has completed and its writes are visible, grid_dep_launch() lets
+// the next pass launch (as the blocks' exit does).  Without the launch attribute
+// both instructions return at once.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_sync() {
-  grid_dep_wait();
-  grid_dep_launch();
-}
 
 template <int U, typename Idx, typename Gather, typename Body>
 __device__ __forceinline__ void walk_bonds(int w, int64_t self, Idx idx, Gather gather, Body body) {
