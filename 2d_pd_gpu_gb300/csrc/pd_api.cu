@@ -264,6 +264,7 @@ void stiffness(const pd_ctx* c, double* c11, double* c12, double* c33);
 Fp64Args fp64_args(pd_ctx* c) {
   Fp64Args a{};
   a.n = a.plate = c->n;
+  a.exit_trigger = c->batch == nullptr;  // (a batch's members run beside one another)
   a.x = c->x; a.vol = c->vol; a.u = c->u; a.v = c->v; a.f = c->f; a.acc = c->acc;
   a.w01 = c->w01; a.w23 = c->w23; a.kinv01 = c->kinv01; a.kinv22 = c->kinv22; a.mt = c->mt; a.hg = c->hg;
   a.bc = c->bc; a.gkind = c->gkind; a.gval = c->gval;
@@ -364,6 +365,7 @@ void stiffness(const pd_ctx* c, double* c11, double* c12, double* c33) {
 pd::MixedArgs mixed_args(pd_ctx* c) {
   pd::MixedArgs a{};
   a.n = c->n;
+  a.exit_trigger = c->batch == nullptr;
   a.npos = c->sell.npos;
   a.x = c->x; a.vol = c->vol;
   a.xs = c->xs; a.vh = c->vh; a.us = c->us; a.vs = c->vsm; a.fs = c->fs; a.ws = c->ws; a.geo = c->geo; a.mh = c->mh;

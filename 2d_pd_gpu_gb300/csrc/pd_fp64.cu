@@ -715,7 +715,7 @@ static void launch_pass(void (*kernel)(Fp64Args), const Fp64Args& a, bool pdl, c
   lc.attrs = at;
   lc.numAttrs = pdl ? 1 : 0;
   Fp64Args b = a;
-  b.exit_trigger = a.n - a.i0 <= kExitTrigger;
+  b.exit_trigger = a.exit_trigger && a.n - a.i0 <= kExitTrigger;
   cudaLaunchKernelEx(&lc, kernel, b);
 }
 

@@ -107,7 +107,7 @@ struct Fp64Args {
   unsigned long long* counters;
   float s2f;                      // s2 rounded to FP32 (converted in a walk, it would take the FP64 pipe per bond)
   int32_t brk;                    // bond breaking on (s_c > 0)
-  int32_t exit_trigger;           // a pass lets the next one launch at its blocks' exit only (set at the launch)
+  int32_t exit_trigger;           // may (in a launch: does) a pass let the next one launch at its blocks' exit only
   int32_t pad;
 };
 
@@ -198,7 +198,7 @@ struct MixedArgs {
   double2* out_v;
   double2* out_f;
   int64_t blk0;
-  int32_t exit_trigger;  // a pass lets the next one launch at its blocks' exit only (set at the launch)
+  int32_t exit_trigger;  // may (in a launch: does) a pass let the next one launch at its blocks' exit only
   int32_t uniform_v;  // every particle's V^ is exactly 1 (pass A leaves the V^ gathers out)
 };
 

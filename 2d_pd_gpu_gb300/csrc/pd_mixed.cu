@@ -1232,7 +1232,8 @@ static void (*pass_a_kernel(const MixedArgs& a, bool breaking))(MixedArgs) {
 // of the blocks that end first, and some SMs run more of them than others (step, us, without / with
 // bonds breaking: 280 x 280 particles 13.5 -> 11.4 / 14.9 -> 12.9, 320 x 320 13.9 -> 12.0 / 16.6 ->
 // 14.7).  Up to two per SM both passes' blocks have their places at once (260 x 260 8.7 us; at the
-// exit 9.4), and a longer pass evens itself out (1M 82 us; 83.6).
+// exit 9.4), and a longer pass evens itself out (1M 82 us; 83.6).  Members of a batch, whose passes
+// run beside one another, let go at their start (16 plates of 67 .. 393 a side: 0.7 % of the call).
 constexpr int64_t kExitFrom = 2 * 152, kExitTo = 3 * 152;
 
 static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_t sm, cudaStream_t s,
@@ -1249,7 +1250,7 @@ static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_
   lc.attrs = at;
   lc.numAttrs = pdl ? 1 : 0;
   MixedArgs b = a;
-  b.exit_trigger = a.nblocks - a.blk0 > kExitFrom && a.nblocks - a.blk0 <= kExitTo;
+  b.exit_trigger = a.exit_trigger && a.nblocks - a.blk0 > kExitFrom && a.nblocks - a.blk0 <= kExitTo;
   cudaLaunchKernelEx(&lc, kernel, b);
 }
 
