@@ -133,21 +133,9 @@ __device__ __forceinline__ float4 w_of(const MixedArgs& a, float2 D1, float2 D2,
 // one addition per warp instead of per particle is most; 160,000 particles 424 -> 184).
 constexpr int kManyLost = 14;
 
-// Pass A's update of the particles that lost bonds (newly > 0 in their lane, p
-// its SELL position, s0 and w its slots): broken count, damage, K^-1, m^ and W^, by the whole warp;
-// D: the lanes' sums in shared memory (the call has few registers to save then).
-// Eight lanes take a particle, four particles at a time: each lane requests
-// four of its first 32 bonds at once and forms their terms, lanes 0 .. 4 each
-// sum one of k11, k12, k22, mx, my over all of them in slot order, and lanes
-// 0 .. 3 share one division: kinv_update_mixed's operations.  One thread alone
-// waits for ~56 dependent loads and ~300 FP64 operations (64 cycles each), and
-// its pass waits for it.
-__device__ __noinline__ void kinv_update_mixed_warp(const MixedArgs& a, int64_t p, int64_t s0, int w, int newly,
-                                                    const float4* D) {
-  constexpr int kPer = 4;  // bonds per lane and round
-  const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
-  unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
-  if (__popc(todo) > kManyLost) {
+__device__ __noinline__ void kinv_update_mixed_lanes(const MixedArgs& a, int64_t p, int64_t s0, int w, int newly,
+                                                     const float4* D) {
+  const int lane = threadIdx.x & 31;
     bool bad = false;
     if (newly > 0) {
       const int64_t i = a.member[p];
@@ -163,8 +151,22 @@ __device__ __noinline__ void kinv_update_mixed_warp(const MixedArgs& a, int64_t 
       atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)all);
       if (nbad) atomicAdd(a.counters + CNT_SINGULAR, (unsigned long long)nbad);
     }
-    return;
-  }
+}
+
+// Pass A's update of the particles that lost bonds (newly > 0 in their lane, p
+// its SELL position, s0 and w its slots): broken count, damage, K^-1, m^ and W^, by the whole warp;
+// D: the lanes' sums in shared memory (the call has few registers to save then).
+// Eight lanes take a particle, four particles at a time: each lane requests
+// four of its first 32 bonds at once and forms their terms, lanes 0 .. 4 each
+// sum one of k11, k12, k22, mx, my over all of them in slot order, and lanes
+// 0 .. 3 share one division: kinv_update_mixed's operations.  One thread alone
+// waits for ~56 dependent loads and ~300 FP64 operations (64 cycles each), and
+// its pass waits for it.
+__device__ __noinline__ void kinv_update_mixed_warp(const MixedArgs& a, int64_t p, int64_t s0, int w, int newly,
+                                                    const float4* D) {
+  constexpr int kPer = 4;  // bonds per lane and round
+  const int lane = threadIdx.x & 31, c = lane & 7, g0 = lane & 24;
+  unsigned todo = __ballot_sync(0xffffffffu, newly > 0);
   while (todo) {
     unsigned rest = todo;  // this lane's particle: that of the (lane / 8)-th lane left to do
     for (int q = lane >> 3; q > 0; --q) rest &= rest - 1;
@@ -405,7 +407,10 @@ __device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, bool 
   if (BREAK && __any_sync(0xffffffffu, newly != 0)) {
     spare[threadIdx.x & 31] = make_float4(D1.x, D1.y, D2.x, D2.y);  // (the warp's staged indices are done with)
     __syncwarp();
-    kinv_update_mixed_warp(a, p, s0, w, newly, spare);
+    if (__popc(__ballot_sync(0xffffffffu, newly != 0)) > kManyLost)
+      kinv_update_mixed_lanes(a, p, s0, w, newly, spare);
+    else
+      kinv_update_mixed_warp(a, p, s0, w, newly, spare);
   }
 }
 
