@@ -293,10 +293,11 @@ __device__ __forceinline__ double sub1(const FpConst& a, double x, double y) { r
 __device__ __forceinline__ double mul1(const FpConst& a, double x, double y) { return fma(x, y, a.neg_zero); }
 
 // Pass A's stretch tests of particle i ahead of its sums, its bonds dealt to the two threads of
-// the pair in turn; broken ones are marked.  Returns the number this thread broke.
+// the pair in turn; broken ones are marked.  Returns the number this thread broke, and the number it left intact.
 constexpr int kTests = 7;  // in flight (1M particles: 2, 4, 7, 14: 712, 696, 684, 682 us per step at 10 blocks per SM)
-__device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, int64_t s0, int w, float2 ui32) {
-  int newly = 0, jn[kTests];
+__device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, int64_t s0, int w, float2 ui32,
+                                          int* intact) {
+  int newly = 0, live = 0, jn[kTests];
   auto indices = [&](int k) {
 #pragma unroll
     for (int q = 0; q < kTests; ++q) jn[q] = k + 2 * q < w ? a.nbr[s0 + (int64_t)(k + 2 * q) * kChunk] : -1;
@@ -317,6 +318,7 @@ __device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, i
     for (int q = 0; q < kTests; ++q) {
       v[q] = j[q] >= 0 ? stretch_fp32(ui32, u[q], e[q], a.s2f) : 1;
       least = min(least, v[q]);
+      live += j[q] >= 0 ? 1 : 0;
     }
     if (least <= 0) {
 #pragma unroll
@@ -329,6 +331,7 @@ __device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, i
       }
     }
   }
+  *intact = live - newly;
   return newly;
 }
 
@@ -336,7 +339,9 @@ __device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, i
 // the sums then need 72 registers instead of 96 and no branch, and other warps' sums keep the FP64
 // pipe busy under the tests (step with bonds breaking, us, 500 x 500 particles 176.7 -> 175.9,
 // 800 x 800 441 -> 435, 1M 683.5 -> 672, 2M 1356 -> 1329).  A smaller plate waits for the tests
-// (400 x 400 117.5 -> 118.1, 100 x 100 15.3 -> 15.9).
+// (400 x 400 117.5 -> 118.1, 100 x 100 15.3 -> 15.9).  Where fewer than 3/4 of a warp's slots hold
+// intact bonds it takes them one by one and leaves out those that no lane has a bond in (1M particles,
+// all but 10 M of 28 M bonds broken: 697 -> 518 us).
 constexpr int64_t kTestsFirst = 250000;
 
 // Pass A of component h of particle i (stretch tests, D, penalty sum, stress,
@@ -364,11 +369,14 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
   const FpConst K = fp_const(a);
   double d1 = 0.0, d2 = 0.0, ah = 0.0;  // row h of D, component h of the penalty sum
   int newly = 0;
+  bool few = false;                             // (the warp's) fewer than 3/4 of the slots hold intact bonds
   constexpr bool TEST = BREAK && !TESTS_FIRST;  // among the sums
   if (BREAK && TESTS_FIRST) {
-    newly = test_bonds(a, i, h, s0, w, ui32);
+    int intact;
+    newly = test_bonds(a, i, h, s0, w, ui32, &intact);
     newly += __shfl_xor_sync(0xffffffffu, newly, 1);
     __syncwarp();  // (the marks are read by both threads)
+    few = 4 * (int)__reduce_add_sync(0xffffffffu, intact) < 3 * (int)__reduce_add_sync(0xffffffffu, w) / 2;
   }
   const float s2 = TEST ? a.s2f : 0.f;
   struct Group {
@@ -429,7 +437,23 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
       if (HG) ah = fma(TEST || on ? g.vj[q] : 1.0, dh, ah);
     }
   };
-  if (most > 0) {
+  if (BREAK && TESTS_FIRST && few) {  // slots that no lane has a bond in cost nothing here
+    const int widest = __reduce_max_sync(0xffffffffu, w);  // (every lane votes)
+    const int64_t mine = ok ? i : a.n - 1;
+#pragma unroll 1
+    for (int k = 0; k < widest; ++k) {
+      const int64_t s = k < w ? s0 + (int64_t)k * kChunk : s0;
+      const int j = k < w ? a.nbr[s] : -1;
+      if (!__any_sync(0xffffffffu, j >= 0)) continue;  // (a vote: predicated off, the sums would keep the pipe busy)
+      const bool on = j >= 0;
+      const int64_t jj = on ? (int64_t)j : mine;
+      const double dh = on ? sub1(K, comp(a.u, jj, h), ui) : -0.0;
+      const double2 t = a.bgeo[s];
+      d1 = fma(dh, on ? t.x : 1.0, d1);
+      d2 = fma(dh, on ? t.y : 1.0, d2);
+      if (HG) ah = fma(on ? a.vol[jj] : 1.0, dh, ah);
+    }
+  } else if (most > 0) {
     Group g0, g1;
     indices(0);
     request(g0, 0);
