@@ -194,7 +194,6 @@ __device__ __noinline__ void kinv_update_warp(const Fp64Args& a, int64_t i, int6
     }
     for (int q = 0; q < 4 && todo; ++q) todo &= todo - 1;
   }
-  __syncwarp();  // the stores above are read by the particles' own lanes
 }
 
 __global__ void __launch_bounds__(kBlock) k_init_geometry(Fp64Args a) {
@@ -475,6 +474,7 @@ __device__ __forceinline__ void pass_a_particle(const Fp64Args& a, int64_t i, in
     if (__any_sync(0xffffffffu, newly != 0)) {
       __syncwarp();  // (other lanes read the marks)
       kinv_update_warp(a, i, s0, w, h == 0 ? newly : 0);
+      __syncwarp();  // (its stores, by either form, are read below by both threads of a pair)
     }
   }
   double2 k01 = make_double2(0.0, 0.0);
