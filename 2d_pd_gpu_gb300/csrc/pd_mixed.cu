@@ -405,7 +405,8 @@ __device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, bool 
   }
   if (live && newly == 0) a.ws[p] = pre.singular ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, D1, D2, pre.geo);
   if (BREAK && __any_sync(0xffffffffu, newly != 0)) {
-    spare[threadIdx.x & 31] = make_float4(D1.x, D1.y, D2.x, D2.y);  // (the warp's staged indices are done with)
+    __syncwarp();  // the warp's staged indices are done with (a vote alone orders no memory)
+    spare[threadIdx.x & 31] = make_float4(D1.x, D1.y, D2.x, D2.y);
     __syncwarp();
     if (__popc(__ballot_sync(0xffffffffu, newly != 0)) > kManyLost)
       kinv_update_mixed_lanes(a, p, s0, w, newly, spare);

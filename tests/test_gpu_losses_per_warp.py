@@ -20,7 +20,7 @@ def _heads(n_heads, lose, pad, seed):
     side = 64
     h = np.stack([np.arange(n_heads) % side, np.arange(n_heads) // side], axis=1) * DX
     ang = 2.0 * np.pi * (np.arange(ANCHORS) / ANCHORS + 0.05 * r.random((n_heads, ANCHORS)))
-    rad = 0.4 * DX * (1.0 + 0.2 * r.random((n_heads, ANCHORS)))
+    rad = 100 * DX * (1.0 + 0.2 * r.random((n_heads, ANCHORS)))  # past the heads, which fill their tiles alone
     anchors = h[:, None, :] + rad[..., None] * np.stack([np.cos(ang), np.sin(ang)], axis=2)
     m = n_heads * (1 + ANCHORS)
     x = np.concatenate([h, anchors.reshape(-1, 2),
@@ -62,3 +62,33 @@ def test_every_number_of_losing_particles_fp64(pdg, po, pad, seed):
     assert np.array_equal(lost, lose) and np.isfinite(sim.f).all()
     assert ctx.counters()["bonds_broken"] == int(lose.sum())
     ctx.close()
+
+
+@pytest.mark.parametrize("part", [0.03, 0.2, 0.4, 0.5, 0.9])  # 32 particles per warp; one lane each from 15 on
+@pytest.mark.parametrize("uniform", [False, True])
+@pytest.mark.parametrize("n_heads", [4096, 4100])
+def test_numbers_of_losing_particles_mixed(pdg, part, uniform, n_heads):
+    """As a context restored after the losses, whose K^-1 is formed afresh from the mask."""
+    r = np.random.default_rng(5)
+    lose = r.random(n_heads) < part
+    x, vol, row_ptr, col, u = _heads(n_heads, lose, 0, 5)
+    if uniform:
+        vol[:] = 1e-9
+    a, b = (pdg.native.Context(pdg.native.default_params(precision=pdg.native.PD_MIXED, E=E_MOD, nu=NU, rho=RHO,
+                                                         dt=1e-7, s_c=S_C, k_hg=1e20)) for _ in range(2))
+    for c in (a, b):
+        c.set_particles(x, vol)
+        c.set_families(row_ptr, col)
+    a.set_state(u, np.zeros_like(u), np.zeros_like(u))
+    a.step(1)
+    mask = a.bond_mask()
+    assert np.array_equal((mask.reshape(-1, ANCHORS) == 0).any(axis=1), lose)
+    assert a.counters()["bonds_broken"] == int(lose.sum())
+    b.restore(a.checkpoint())
+    for c in (a, b):
+        c.step(2)
+    for p, q in zip(a.state(), b.state()):
+        assert np.isfinite(p).all() and np.array_equal(p, q)
+    assert np.array_equal(a.bond_mask(), b.bond_mask()) and np.array_equal(a.damage(), b.damage())
+    a.close()
+    b.close()
