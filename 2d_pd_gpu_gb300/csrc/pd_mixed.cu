@@ -1055,6 +1055,7 @@ __global__ void __launch_bounds__(kHaloBlock) k_batch_persistent_mixed(const Mix
     ok = batch_phase_mixed<-1>(plates, tiles, ntiles, 1, sm, bars);
     if (!ok) break;
     if (!grid_sync(bar, nb, lim)) return;
+    fence_global_for_copies();  // (pass A marks broken bonds in the indices that the later passes stage)
     ok = batch_phase_mixed<-1>(plates, tiles, ntiles, s + 1 < nsteps ? 2 : 3, sm, bars);
   }
   if (!ok && threadIdx.x == 0) atomicExch(&bar->err, 1);  // releases the other blocks' barrier waits

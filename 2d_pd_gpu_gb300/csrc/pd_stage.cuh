@@ -53,6 +53,12 @@ __device__ __forceinline__ void stage_issue(void* dst, const void* src, uint32_t
       : "memory");
 }
 
+// Orders global writes that this thread has seen (or made) before the bulk copies it
+// issues after: for a kernel whose own earlier phases wrote what it now stages.
+__device__ __forceinline__ void fence_global_for_copies() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+
 // Any thread, after the issuing thread's stage_issue is ordered before it
 // (same thread, __syncwarp or __syncthreads).  False if the copy did not
 // land in time (after one more bounded wait for it).
