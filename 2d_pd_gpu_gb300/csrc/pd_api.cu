@@ -306,15 +306,24 @@ pd::BondAssoc ba_args(pd_ctx* c) {
   return b;
 }
 
-// Buffers and reverse-slot index of the bond-associated mode, and its
-// per-bond constants for the current weights (recomputed on every call: the
-// parameters may have changed).
+// The bond-associated tables and reverse slots hold the families' intact bonds as they were
+// when they were formed.  They are formed again when the weights are set (whatever
+// happened to the mask before) and, while they are, when a reset or a restore changes the mask.
+void reform_ba(pd_ctx* c) {
+  if (!bond_assoc(c) || !c->tb) return;
+  pd::launch_ba_reverse(fp64_args(c), ba_args(c), c->stream);
+  pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
+}
+
+// Buffers of the bond-associated mode, its reverse-slot index over the intact
+// bonds and its per-bond constants for the current weights (formed again on
+// every call: the parameters and the mask may have changed).
 int ensure_ba(pd_ctx* c) {
   if (!bond_assoc(c) || !c->has_families) return PD_OK;
   if (c->max_family > 64) return fail(c, PD_ERR_CAPACITY, "bond-associated mode: families are limited to 64 bonds");
   const size_t ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
-  if (c->tb) {
-    pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
+  if (c->tb) {  // (the mask may have changed under classic weights, too: steps, a reset, a restore)
+    reform_ba(c);
     PD_CK(c, cudaGetLastError());
     return PD_OK;
   }
@@ -342,14 +351,6 @@ int ensure_ba(pd_ctx* c) {
   PD_CK(c, cudaStreamSynchronize(c->stream));
   if (err & pd::ERR_ASYMMETRIC) return fail(c, PD_ERR_ARG, "bond-associated mode needs symmetric families");
   return PD_OK;
-}
-
-// The bond-associated tables and reverse slots hold the families' intact bonds as they were
-// when they were formed: after a change of the mask (a reset or a restore) they are formed again.
-void reform_ba(pd_ctx* c) {
-  if (!bond_assoc(c) || !c->tb) return;
-  pd::launch_ba_reverse(fp64_args(c), ba_args(c), c->stream);
-  pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
 }
 
 bool mixed(const pd_ctx* c) { return c->p.precision == PD_MIXED; }

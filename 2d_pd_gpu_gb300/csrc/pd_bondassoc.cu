@@ -444,7 +444,8 @@ __global__ void k_ba_bonds(Fp64Args a, BondAssoc b, int64_t nslots) {
   b.ex[s] = make_double2(exp(b.n1 * (l * b.inv_wlen)), exp(-b.n1 * (l * b.inv_wlen)));
 }
 
-// rslot[s] = slot of (j, i) in j's SELL rows, for every slot s = (i, j).
+// rslot[s] = slot of (j, i) in j's SELL rows, for every slot s = (i, j) of an intact bond;
+// itself for the others (every entry is a slot).
 __global__ void k_ba_reverse(Fp64Args a, BondAssoc b, unsigned long long* counters) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -454,7 +455,10 @@ __global__ void k_ba_reverse(Fp64Args a, BondAssoc b, unsigned long long* counte
   for (int k = 0; k < w; ++k) {
     const int64_t s = s0 + (int64_t)k * kChunk;
     const int j = a.nbr[s];
-    if (j < 0) continue;
+    if (j < 0) {
+      b.rslot[s] = s;
+      continue;
+    }
     const int64_t cj = (int64_t)j >> 5;
     const int wj = a.chunk_w[cj];
     const int64_t sj0 = a.chunk_base[cj] + (j & 31);
