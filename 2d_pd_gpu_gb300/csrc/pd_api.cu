@@ -259,6 +259,9 @@ void* mapped_host(const void* p) {
   return at.devicePointer;
 }
 
+// The kernels read and write the state of a particle in host memory as one 16-byte element.
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 void stiffness(const pd_ctx* c, double* c11, double* c12, double* c33);
 
 Fp64Args fp64_args(pd_ctx* c) {
@@ -1769,20 +1772,29 @@ int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_
   if (!u_in || !v_in || !f_in || !u_out || !v_out || !f_out) return fail(c, PD_ERR_ARG, "pd_step_host: NULL buffer");
   if (c->n == 0) return PD_OK;
   PD_CK(c, cudaSetDevice(c->p.device));
-  if (mixed(c)) {
-    if (!mapped_host(u_in) || !mapped_host(v_in) || !mapped_host(f_in) || !mapped_host(u_out) ||
-        !mapped_host(v_out) || !mapped_host(f_out))
+  const double* hin[3] = {u_in, v_in, f_in};
+  double* hout[3] = {u_out, v_out, f_out};
+  const double2* from[3];
+  double2* to[3];
+  bool direct = true;
+  for (int k = 0; k < 3; ++k) {
+    from[k] = static_cast<const double2*>(mapped_host(hin[k]));
+    to[k] = static_cast<double2*>(mapped_host(hout[k]));
+    if (!from[k] || !to[k])
       return fail(c, PD_ERR_ARG, "pd_step_host: buffers must be page-locked host memory (pd_host_alloc)");
+    // (the mixed pipeline takes its input by copies alone)
+    direct = direct && aligned16(to[k]) && (aligned16(from[k]) || (mixed(c) && c->n >= kPipelineFromMixed));
+  }
+  if (!direct) {  // a buffer that begins inside a 16-byte element: by copies
+    int rc = pd_set_state(c, u_in, v_in, f_in);
+    if (rc == PD_OK) rc = pd_step(c, nsteps);
+    if (rc != PD_OK && rc != PD_ERR_SINGULAR) return rc;
+    const int rg = pd_get_state(c, u_out, v_out, f_out);
+    return rg != PD_OK ? rg : rc;
+  }
+  if (mixed(c)) {
     if (c->n < kPipelineFromMixed) {
-      const double2* in[3];
-      double2* out[3];
-      const double* hin[3] = {u_in, v_in, f_in};
-      double* hout[3] = {u_out, v_out, f_out};
-      for (int k = 0; k < 3; ++k) {
-        in[k] = static_cast<const double2*>(mapped_host(hin[k]));
-        out[k] = static_cast<double2*>(mapped_host(hout[k]));
-      }
-      const int rs = small_host_step(c, nsteps, in, out);
+      const int rs = small_host_step(c, nsteps, from, to);
       if (rs != PD_OK) return rs;
     } else {
       const int rp = plan_slabs_mixed(c);
@@ -1794,15 +1806,13 @@ int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_
     c->steps += nsteps;
     return check_after_step(c);
   }
-  Fp64Args in = fp64_args(c), out = fp64_args(c);
-  in.in_u = static_cast<const double2*>(mapped_host(u_in));
-  in.in_v = static_cast<const double2*>(mapped_host(v_in));
-  in.in_f = static_cast<const double2*>(mapped_host(f_in));
-  out.out_u = static_cast<double2*>(mapped_host(u_out));
-  out.out_v = static_cast<double2*>(mapped_host(v_out));
-  out.out_f = static_cast<double2*>(mapped_host(f_out));
-  if (!in.in_u || !in.in_v || !in.in_f || !out.out_u || !out.out_v || !out.out_f)
-    return fail(c, PD_ERR_ARG, "pd_step_host: buffers must be page-locked host memory (pd_host_alloc)");
+  Fp64Args in = fp64_args(c), out = in;
+  in.in_u = from[0];
+  in.in_v = from[1];
+  in.in_f = from[2];
+  out.out_u = to[0];
+  out.out_v = to[1];
+  out.out_f = to[2];
   cudaStream_t s = c->stream;
   const Fp64Args plain = fp64_args(c);
   const bool brk = c->p.s_c > 0.0;
@@ -1814,8 +1824,6 @@ int pd_step_host(pd_ctx* c, int32_t nsteps, const double* u_in, const double* v_
       pd::launch_ba_pass_b(last ? out : plain, ba_args(c), last ? 0 : 1, s);
     }
   } else if (c->n < kPipelineFrom) {
-    const double2* from[3] = {in.in_u, in.in_v, in.in_f};
-    double2* to[3] = {out.out_u, out.out_v, out.out_f};
     const int rs = small_host_step(c, nsteps, from, to);
     if (rs != PD_OK) return rs;
   } else {
@@ -1849,17 +1857,21 @@ int pd_compute_velocity(pd_ctx* c, const double* u, double* velocity, double* ac
   PD_CK(c, cudaSetDevice(c->p.device));
   const size_t b = (size_t)c->n * sizeof(double2);
   cudaStream_t s = c->stream;
-  if (!bond_assoc(c) && mapped_host(u) && mapped_host(velocity) && mapped_host(acce) && mapped_host(netF)) {
+  const void* host[4] = {u, velocity, acce, netF};
+  void* dev[4] = {};
+  bool direct = !bond_assoc(c);
+  for (int k = 0; direct && k < 4; ++k) direct = (dev[k] = mapped_host(host[k])) != nullptr && aligned16(dev[k]);
+  if (direct) {
     // page-locked buffers (pd_host_alloc): pd_step_host's slab pipeline, the
     // copies in overlapping pass A and each slab's pass B writing its results
     // back while later slabs compute; the same results as the staged call
     Fp64Args out = fp64_args(c);
-    out.out_v = static_cast<double2*>(mapped_host(velocity));
-    out.out_a = static_cast<double2*>(mapped_host(acce));
-    out.out_f = static_cast<double2*>(mapped_host(netF));
+    out.out_v = static_cast<double2*>(dev[1]);
+    out.out_a = static_cast<double2*>(dev[2]);
+    out.out_f = static_cast<double2*>(dev[3]);
     if (c->n < kPipelineFrom) {  // (too small for the pipeline: one import of u, velocity and acce)
       Fp64Args in = fp64_args(c);
-      in.in_u = static_cast<const double2*>(mapped_host(u));
+      in.in_u = static_cast<const double2*>(dev[0]);
       in.in_v = out.out_v;
       in.in_a = out.out_a;
       pd::launch_shadow_fp64(in, s);

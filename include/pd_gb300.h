@@ -223,7 +223,8 @@ int pd_step(pd_ctx* ctx, int32_t nsteps);
  * same, through the mixed form's own slabs of spatial tiles.  Small plates
  * (FP64 below 220,000 particles, mixed below 900,000) go without the slabs:
  * the first kernel reads the buffers and the last one writes them.  In and
- * out may be the same buffers.
+ * out may be the same buffers.  Buffers that do not begin on 16 bytes (a view
+ * into a larger one) are taken too, by pd_set_state + pd_step + pd_get_state.
  * Synchronous; the device state and the outputs are those of pd_set_state +
  * pd_step + pd_get_state, bit for bit. */
 int pd_step_host(pd_ctx* ctx, int32_t nsteps, const double* u_in, const double* v_in, const double* f_in,
@@ -240,7 +241,7 @@ int pd_synchronize(pd_ctx* ctx);
  * velocity += 0.5 (acce + f/rho) dt, acce = f/rho and netF = f.  Device
  * buffers stay allocated between calls.  The bond mask persists across calls
  * and breaks bonds as in pd_step when s_c > 0.  When all four buffers are
- * page-locked (pd_host_alloc) and the context is in the plain mode, the call
+ * page-locked (pd_host_alloc), begin on 16 bytes and the context is in the plain mode, the call
  * runs as pd_step_host's first and last step do: from 220,000 particles on its
  * slab pipeline (the copies in overlap the first pass, and each slab's results
  * go back while later slabs compute), below that the kernels read and write the
