@@ -167,6 +167,13 @@ cudaError_t copy_sync(void* dst, const void* src, size_t bytes, cudaMemcpyKind k
   return e;
 }
 
+void drop_mazars_table(pd_ctx* c) {
+  dfree(c->mz_tt);
+  dfree(c->mz_kq0);
+  dfree(c->mz_kq1);
+  c->mz_table_ok = c->mz_table_none = false;
+}
+
 void free_families(pd_ctx* c) {
   dfree(c->row_ptr);
   dfree(c->col);
@@ -181,10 +188,7 @@ void free_families(pd_ctx* c) {
   dfree(c->mz_thr);
   dfree(c->mz_bd);
   dfree(c->mz_status);
-  dfree(c->mz_tt);
-  dfree(c->mz_kq0);
-  dfree(c->mz_kq1);
-  c->mz_table_ok = c->mz_table_none = false;
+  drop_mazars_table(c);
   dfree(c->halo.visit);
   dfree(c->halo.loc);
   dfree(c->halo.loc0);
@@ -353,6 +357,48 @@ int ensure_ba(pd_ctx* c) {
   PD_CK(c, cudaMemcpyAsync(&err, c->counters + pd::CNT_ERROR, sizeof(err), cudaMemcpyDeviceToHost, c->stream));
   PD_CK(c, cudaStreamSynchronize(c->stream));
   if (err & pd::ERR_ASYMMETRIC) return fail(c, PD_ERR_ARG, "bond-associated mode needs symmetric families");
+  return PD_OK;
+}
+
+pd::MazarsArgs mazars_args(pd_ctx* c) {
+  pd::MazarsArgs m{};
+  m.kappa0 = c->mz.kappa0;
+  m.a_t = c->mz.a_t;
+  m.b_t = c->mz.b_t;
+  m.a_c = c->mz.a_c;
+  m.b_c = c->mz.b_c;
+  m.thr = c->mz_thr;
+  m.bd = c->mz_bd;
+  m.status = c->mz_status;
+  if (c->mz_table_ok) {
+    m.tt = c->mz_tt;
+    m.kq0 = c->mz_kq0;
+    m.kq1 = c->mz_kq1;
+  }
+  return m;
+}
+
+// The bond-associated update's weight table (16 KB per particle) for the current parameters,
+// formed with the history (pd_mazars_init) and when the parameters are set.  Where it would
+// take more than a quarter of the free memory, the updates evaluate the weights themselves.
+int ensure_mazars_table(pd_ctx* c) {
+  if (!c->mz_thr || !bond_assoc(c) || c->mz_table_ok || c->mz_table_none || c->n == 0) return PD_OK;
+  const size_t bytes = (size_t)c->n * 1024 * sizeof(double2), ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
+  if (!c->mz_kq1) {
+    size_t free_b = 0, total_b = 0;
+    bool ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes / 3 < free_b / 12;
+    ok = ok && cudaMalloc(&c->mz_tt, bytes) == cudaSuccess && cudaMalloc(&c->mz_kq0, ns * sizeof(double2)) == cudaSuccess &&
+         cudaMalloc(&c->mz_kq1, ns * sizeof(double2)) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      drop_mazars_table(c);
+      c->mz_table_none = true;
+      return PD_OK;
+    }
+  }
+  c->mz_table_ok = true;
+  pd::launch_mazars_table(fp64_args(c), ba_args(c), mazars_args(c), c->stream);
+  PD_CK(c, cudaGetLastError());
   return PD_OK;
 }
 
@@ -624,6 +670,8 @@ int pd_set_params(pd_ctx* c, const pd_params* p) {
     int rc2 = upload_gvel(c);
     if (rc2 != PD_OK) return rc2;
     rc2 = ensure_ba(c);
+    if (rc2 != PD_OK) return rc2;
+    rc2 = ensure_mazars_table(c);
     if (rc2 != PD_OK) return rc2;
   }
   return PD_OK;
@@ -1014,54 +1062,6 @@ int pd_step(pd_ctx* c, int32_t nsteps) {
 }
 
 // ---- Mazars damage
-namespace {
-
-pd::MazarsArgs mazars_args(pd_ctx* c) {
-  pd::MazarsArgs m{};
-  m.kappa0 = c->mz.kappa0;
-  m.a_t = c->mz.a_t;
-  m.b_t = c->mz.b_t;
-  m.a_c = c->mz.a_c;
-  m.b_c = c->mz.b_c;
-  m.thr = c->mz_thr;
-  m.bd = c->mz_bd;
-  m.status = c->mz_status;
-  if (c->mz_table_ok) {
-    m.tt = c->mz_tt;
-    m.kq0 = c->mz_kq0;
-    m.kq1 = c->mz_kq1;
-  }
-  return m;
-}
-
-bool bond_associated(const pd_ctx* c) { return c->p.n1 != 0.0 || c->p.n2 != 0.0; }
-
-// The bond-associated update's weight table (16 KB per particle), formed for the current
-// parameters on first use.  Where it would take more than a quarter of the free memory, the
-// updates evaluate the weights themselves.
-void ensure_mazars_table(pd_ctx* c) {
-  if (!bond_associated(c) || c->mz_table_ok || c->mz_table_none || c->n == 0) return;
-  const size_t bytes = (size_t)c->n * 1024 * sizeof(double2), ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
-  if (!c->mz_kq1) {
-    size_t free_b = 0, total_b = 0;
-    bool ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes / 3 < free_b / 12;
-    ok = ok && cudaMalloc(&c->mz_tt, bytes) == cudaSuccess && cudaMalloc(&c->mz_kq0, ns * sizeof(double2)) == cudaSuccess &&
-         cudaMalloc(&c->mz_kq1, ns * sizeof(double2)) == cudaSuccess;
-    if (!ok) {
-      cudaGetLastError();
-      dfree(c->mz_tt);
-      dfree(c->mz_kq0);
-      dfree(c->mz_kq1);
-      c->mz_table_none = true;
-      return;
-    }
-  }
-  c->mz_table_ok = true;
-  pd::launch_mazars_table(fp64_args(c), ba_args(c), mazars_args(c), c->stream);
-}
-
-}  // namespace
-
 void pd_mazars_default_params(pd_mazars_params* p) {
   if (!p) return;
   p->kappa0 = 3.0 / 3.5e4;
@@ -1078,7 +1078,7 @@ int pd_mazars_init(pd_ctx* c, const pd_mazars_params* p) {
   if (!(p->kappa0 >= 0.0) || !std::isfinite(p->kappa0) || !std::isfinite(p->a_t) || !std::isfinite(p->b_t) ||
       !std::isfinite(p->a_c) || !std::isfinite(p->b_c))
     return fail(c, PD_ERR_ARG, "invalid Mazars parameters");
-  if (bond_associated(c) && c->max_family > 64)
+  if (bond_assoc(c) && c->max_family > 64)
     return fail(c, PD_ERR_CAPACITY, "bond-associated Mazars damage: families are limited to 64 bonds");
   PD_CK(c, cudaSetDevice(c->p.device));
   PD_CK(c, cudaStreamSynchronize(c->stream));
@@ -1089,6 +1089,8 @@ int pd_mazars_init(pd_ctx* c, const pd_mazars_params* p) {
   c->mz = *p;
   pd::launch_mazars_reset(c->sell.nslots, c->n, mazars_args(c), c->stream);
   PD_CK(c, cudaGetLastError());
+  const int rt = ensure_mazars_table(c);
+  if (rt != PD_OK) return rt;
   PD_CK(c, cudaStreamSynchronize(c->stream));
   return PD_OK;
 }
@@ -1098,8 +1100,7 @@ int pd_mazars_update(pd_ctx* c) {
   if (!c->mz_thr) return fail(c, PD_ERR_ORDER, "pd_mazars_init first");
   PD_CK(c, cudaSetDevice(c->p.device));
   const pd::BondAssoc ba = ba_args(c);
-  ensure_mazars_table(c);
-  pd::launch_mazars_update(fp64_args(c), bond_associated(c) ? &ba : nullptr, mazars_args(c), c->stream);
+  pd::launch_mazars_update(fp64_args(c), bond_assoc(c) ? &ba : nullptr, mazars_args(c), c->stream);
   PD_CK(c, cudaGetLastError());
   return PD_OK;
 }
@@ -1275,6 +1276,7 @@ int pd_checkpoint_load(pd_ctx* c, const void* buf, int64_t bytes) {
     dfree(c->mz_thr);
     dfree(c->mz_bd);
     dfree(c->mz_status);
+    drop_mazars_table(c);
   }
   c->mz = h.mz;
   int64_t need = 0;
