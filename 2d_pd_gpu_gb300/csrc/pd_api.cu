@@ -62,6 +62,7 @@ struct pd_ctx {
   double2* ba_kq0 = nullptr;  // K_b^-1 with its det-guard flag
   double2* ba_kq1 = nullptr;
   double* ba_wfull = nullptr;  // and, per particle, its weight matrix
+  double* ba_wtri = nullptr;   // or its lower triangle
   double* ba_rv = nullptr;    // and 1 / its family's volume
   bool mask_cut = false;      // bonds may have broken since the last reset (under earlier parameters)
   int32_t max_family = 0;
@@ -206,6 +207,7 @@ void free_families(pd_ctx* c) {
   dfree(c->ba_kq0);
   dfree(c->ba_kq1);
   dfree(c->ba_wfull);
+  dfree(c->ba_wtri);
   dfree(c->ba_rv);
   c->sell = pd::SellLayout{};
   c->slab_bnd.clear();
@@ -308,9 +310,23 @@ pd::BondAssoc ba_args(pd_ctx* c) {
   b.kq0 = c->ba_kq0;
   b.kq1 = c->ba_kq1;
   b.wfull = c->ba_wfull;
+  b.wtri = c->ba_wtri;
   b.max_family = c->max_family;
   b.rv = c->ba_rv;
   return b;
+}
+
+// A table that only saves evaluating its entries again takes at most a quarter of the free
+// memory: the rest is left to other contexts and to the program.
+template <typename T>
+bool alloc_table(T** p, size_t count) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && count <= free_b / (4 * sizeof(T)) &&
+      cudaMalloc(p, count * sizeof(T)) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
 }
 
 // The bond-associated tables and reverse slots hold the families' intact bonds as they were
@@ -342,10 +358,12 @@ int ensure_ba(pd_ctx* c) {
   if (!c->ba_rv) PD_CK(c, cudaMalloc(&c->ba_rv, (size_t)(c->n > 0 ? c->n : 1) * sizeof(double)));
   if (!c->rslot) PD_CK(c, cudaMalloc(&c->rslot, ns * sizeof(int64_t)));
   PD_CK(c, cudaMalloc(&c->tb, ns * sizeof(double2)));
-  // (8 KB per particle: where it does not fit, the passes evaluate the weights; the same results)
-  if (!c->ba_wfull &&
-      cudaMalloc(&c->ba_wfull, (size_t)(c->n > 0 ? c->n : 1) * (size_t)pd::kBaFull * sizeof(double)) != cudaSuccess) {
-    c->ba_wfull = nullptr;
+  // the weight matrices, 8 KB per particle; where they would take too much, their lower triangles
+  // (4 KB) if these can be had at all; else the passes evaluate the weights: the same results
+  const size_t np = (size_t)(c->n > 0 ? c->n : 1);
+  if (!c->ba_wfull && !c->ba_wtri && !alloc_table(&c->ba_wfull, np * (size_t)pd::kBaFull) &&
+      cudaMalloc(&c->ba_wtri, np * (size_t)pd::kBaTri * sizeof(double)) != cudaSuccess) {
+    c->ba_wtri = nullptr;
     cudaGetLastError();
   }
   pd::launch_ba_bonds(fp64_args(c), ba_args(c), c->sell.nslots, c->stream);
@@ -379,18 +397,13 @@ pd::MazarsArgs mazars_args(pd_ctx* c) {
 }
 
 // The bond-associated update's weight table (16 KB per particle) for the current parameters,
-// formed with the history (pd_mazars_init) and when the parameters are set.  Where it would
-// take more than a quarter of the free memory, the updates evaluate the weights themselves.
+// formed with the history (pd_mazars_init) and when the parameters are set; without it the
+// updates evaluate the weights.
 int ensure_mazars_table(pd_ctx* c) {
   if (!c->mz_thr || !bond_assoc(c) || c->mz_table_ok || c->mz_table_none || c->n == 0) return PD_OK;
-  const size_t bytes = (size_t)c->n * 1024 * sizeof(double2), ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
+  const size_t ns = (size_t)(c->sell.nslots > 0 ? c->sell.nslots : 1);
   if (!c->mz_kq1) {
-    size_t free_b = 0, total_b = 0;
-    bool ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes / 3 < free_b / 12;
-    ok = ok && cudaMalloc(&c->mz_tt, bytes) == cudaSuccess && cudaMalloc(&c->mz_kq0, ns * sizeof(double2)) == cudaSuccess &&
-         cudaMalloc(&c->mz_kq1, ns * sizeof(double2)) == cudaSuccess;
-    if (!ok) {
-      cudaGetLastError();
+    if (!alloc_table(&c->mz_tt, (size_t)c->n * 1024) || !alloc_table(&c->mz_kq0, ns) || !alloc_table(&c->mz_kq1, ns)) {
       drop_mazars_table(c);
       c->mz_table_none = true;
       return PD_OK;

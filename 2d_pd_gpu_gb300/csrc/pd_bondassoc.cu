@@ -165,21 +165,30 @@ __global__ void __launch_bounds__(32 * kBaWarps) k_ba_pass_a(Fp64Args a, BondAss
   for (int o = 16; o; o >>= 1) lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
   wf.direct = !(fabs(b.n1) * lmax * b.inv_wlen < 600.0);
   __syncwarp();
-  const bool tri = n <= 32 && b.wfull != nullptr;
-  if (tri) {
-    double* wt = b.wfull + i * kBaFull;
-    if (KTAB) {  // pair p = k (k + 1) / 2 + q, q <= k, of the lower triangle, evaluated and kept
-      const int npair = n * (n + 1) / 2;
-      for (int p = lane; p < npair; p += 32) {
-        int k = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
-        if ((k + 1) * (k + 2) / 2 <= p) ++k;
-        if (k * (k + 1) / 2 > p) --k;
-        const int q = p - k * (k + 1) / 2;
-        const double wqk = wf(F, q, k);
-        F.wrow[k][q] = wqk;
-        F.wrow[q][k] = wqk;
+  const bool tri = n <= 32 && (b.wfull || b.wtri);
+  if (tri && (KTAB || !b.wfull)) {  // pair p = k (k + 1) / 2 + q, q <= k, of the lower triangle
+    const int npair = n * (n + 1) / 2;
+    double* wt = b.wtri + i * kBaTri;
+    for (int p = lane; p < npair; p += 32) {
+      int k = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
+      if ((k + 1) * (k + 2) / 2 <= p) ++k;
+      if (k * (k + 1) / 2 > p) --k;
+      const int q = p - k * (k + 1) / 2;
+      double wqk;
+      if (KTAB) {  // evaluated and kept
+        wqk = wf(F, q, k);
+        if (!b.wfull) wt[p] = wqk;
+      } else {
+        wqk = wt[p];
       }
-      __syncwarp();
+      F.wrow[k][q] = wqk;
+      F.wrow[q][k] = wqk;
+    }
+    __syncwarp();
+  }
+  if (tri && b.wfull) {
+    double* wt = b.wfull + i * kBaFull;
+    if (KTAB) {
       for (int k = 0; k < 32; ++k) wt[k * 32 + lane] = k < n && lane < n ? F.wrow[k][lane] : 0.0;
     } else {
       for (int k = 0; k < n; ++k) F.wrow[k][lane] = wt[k * 32 + lane];

@@ -121,10 +121,11 @@ struct BondAssoc {
   double2* kq0;    // per bond slot: K_b^-1 (q11, q12)
   double2* kq1;    // per bond slot: (q22, 1 if K_b fails the det guard else 0)
   double* wfull;   // per particle with <= 32 bonds: its weight matrix, w(q, k) at [k][q] (kBaFull doubles); or null
+  double* wtri;    // or its lower triangle, w(q, k), q <= k, at k (k + 1) / 2 + q (kBaTri doubles); or null
   double* rv;      // per particle: 1 / its family's volume
   int32_t max_family, pad;
 };
-constexpr int64_t kBaFull = 32 * 32;
+constexpr int64_t kBaFull = 32 * 32, kBaTri = 32 * 33 / 2;
 
 // Mazars damage (pd_mazars.cu): law constants and per-slot history.
 struct MazarsArgs {
