@@ -87,8 +87,8 @@ struct pd_ctx {
   // counters (device) + host mirror of steps
   unsigned long long* counters = nullptr;
   int64_t steps = 0;
-  // graphs per step count
-  std::map<int32_t, cudaGraphExec_t> graphs;
+  // graphs per step count and place (graph_key)
+  std::map<int64_t, cudaGraphExec_t> graphs;
   // drop-in staging (pinned)
   std::vector<void*> scratch;
   // batch membership (pd_batch_add)
@@ -148,6 +148,10 @@ void clear_batch_graphs(pd_batch* b) {
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->graphs.clear();
 }
+
+// A member of a batch and the same context alone launch their passes differently
+// (Fp64Args, MixedArgs: exit_trigger), so each has graphs of its own.
+int64_t graph_key(const pd_ctx* c, int32_t nsteps) { return 2 * (int64_t)nsteps + (c->batch != nullptr); }
 
 // Captured kernel arguments are stale: drop the graphs (and the batch tables).
 void clear_graphs(pd_ctx* c) {
@@ -1032,7 +1036,8 @@ int check_after_step(pd_ctx* c) {
 
 // The graph of nsteps steps of c (enqueue_steps' launches), captured on c's stream on first use.
 int step_graph(pd_ctx* c, int32_t nsteps, cudaGraphExec_t* out) {
-  auto it = c->graphs.find(nsteps);
+  const int64_t key = graph_key(c, nsteps);
+  auto it = c->graphs.find(key);
   if (it == c->graphs.end()) {
     cudaGraph_t g;
     PD_CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -1047,7 +1052,7 @@ int step_graph(pd_ctx* c, int32_t nsteps, cudaGraphExec_t* out) {
       for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
       c->graphs.clear();
     }
-    it = c->graphs.emplace(nsteps, ge).first;
+    it = c->graphs.emplace(key, ge).first;
   }
   *out = it->second;
   return PD_OK;
@@ -1713,11 +1718,12 @@ static cudaError_t enqueue_host_step_mixed(pd_ctx* c, int32_t nsteps, const doub
 constexpr int64_t kPipelineFrom = 220000, kPipelineFromMixed = 900000;
 
 // The graph of kInnerSteps steps between an import and the last step: pass A,
-// pass B + the next drift, each.  One per context (under the key -kInnerSteps of
-// its graphs), whatever the callers' step counts.
+// pass B + the next drift, each.  One per context and place (under the step count
+// -kInnerSteps), whatever the callers' step counts.
 constexpr int32_t kInnerSteps = 16;
 static int inner_graph(pd_ctx* c, cudaGraphExec_t* out) {
-  const auto it = c->graphs.find(-kInnerSteps);
+  const int64_t key = graph_key(c, -kInnerSteps);
+  const auto it = c->graphs.find(key);
   if (it != c->graphs.end()) {
     *out = it->second;
     return PD_OK;
@@ -1734,7 +1740,7 @@ static int inner_graph(pd_ctx* c, cudaGraphExec_t* out) {
   e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return cuda_fail(c, e, "graph instantiate");
-  c->graphs.emplace(-kInnerSteps, *out);
+  c->graphs.emplace(key, *out);
   return PD_OK;
 }
 
