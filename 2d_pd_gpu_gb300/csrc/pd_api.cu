@@ -295,7 +295,7 @@ Fp64Args fp64_args(pd_ctx* c) {
   a.neg_one = -1.0;
   a.neg_zero = -0.0;
   a.s2 = c->p.s_c > 0.0 ? c->p.s_c * (2.0 + c->p.s_c) : INFINITY;
-  a.s2f = (float)a.s2;
+  a.s2f = a.s2 >= 1e-30 && a.s2 <= 1e6 ? (float)a.s2 : 0.0f;  // (stretch_fp32: its range)
   a.damage_fail = c->p.damage_fail;
   a.counters = c->counters;
   a.brk = c->p.s_c > 0.0;

@@ -248,8 +248,11 @@ __global__ void __launch_bounds__(kBlock) k_shadow(Fp64Args a) {
 // f.(2 xi + f) by at most sum delta_c (2 S_c + delta_c), and xi's and the
 // evaluation's rounding add at most 4 * 2^-24 sum |f_c| S_c; the limit's own
 // relative error is below 6 * 2^-24.  The margins taken (6.0e-8, 3e-7 and 1e-6)
-// are above these and the FP64 evaluation's ~1e-15.  Limits where FP32 products
-// could underflow or overflow, and any infinity or NaN, leave it to FP64.
+// are above these and the FP64 evaluation's ~1e-15.  These are relative errors, which
+// hold while nothing that counts is below FP32's normal range (s2 itself, |xi|^2, the
+// limit): limits outside 1e-30 .. 1e30 leave it to FP64, so do infinities and NaN, and
+// outside 1e-30 <= s2 <= 1e6 the host passes s2 = 0, a limit of 0.  Inside, |xi|^2 >=
+// 1e-36, and what underflows elsewhere is below 1e-36 of a limit's 1e-30.
 // A test that bounds |d| alone leaves every rotating or compressed bond to FP64
 // too, which in the few warps of a fracture zone is what the whole pass waits
 // for (300 x 300 plate with bonds breaking: see k_pass_a).

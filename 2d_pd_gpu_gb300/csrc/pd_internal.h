@@ -105,7 +105,7 @@ struct Fp64Args {
   double one, neg_one, neg_zero;  // 1, -1, -0 (add1, sub1, mul1)
   double s2;                      // stretch limit factor (1 + s_c)^2 - 1 = s_c (2 + s_c)
   unsigned long long* counters;
-  float s2f;                      // s2 rounded to FP32 (converted in a walk, it would take the FP64 pipe per bond)
+  float s2f;                      // s2 in FP32, 0 outside stretch_fp32's range (converted in a walk: FP64 pipe per bond)
   int32_t brk;                    // bond breaking on (s_c > 0)
   int32_t exit_trigger;           // may (in a launch: does) a pass let the next one launch at its blocks' exit only
   int32_t pad;
