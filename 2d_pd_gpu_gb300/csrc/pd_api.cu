@@ -66,6 +66,7 @@ struct pd_ctx {
   double* ba_rv = nullptr;    // and 1 / its family's volume
   bool mask_cut = false;      // bonds may have broken since the last reset (under earlier parameters)
   int32_t max_family = 0;
+  int32_t nsm = 0;  // SMs of the device
   // pd_step_host's copy / compute pipeline (streams and events, see plan_slabs)
   cudaStream_t io[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   std::vector<cudaStream_t> ps;  // pd_step_host: one stream per slab's pass A, then one per slab's pass B
@@ -433,6 +434,7 @@ pd::MixedArgs mixed_args(pd_ctx* c) {
   pd::MixedArgs a{};
   a.n = c->n;
   a.exit_trigger = c->batch == nullptr;
+  a.nsm = c->nsm;
   a.npos = c->sell.npos;
   a.x = c->x; a.vol = c->vol;
   a.xs = c->xs; a.vh = c->vh; a.us = c->us; a.vs = c->vsm; a.fs = c->fs; a.ws = c->ws; a.geo = c->geo; a.mh = c->mh;
@@ -632,6 +634,7 @@ int pd_create(const pd_params* p, pd_ctx** out) {
   }
   c->p = *p;
   cudaError_t e = cudaSetDevice(p->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, p->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&c->counters, pd::CNT_N * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->counters, 0, pd::CNT_N * sizeof(unsigned long long), c->stream);

@@ -200,6 +200,7 @@ struct MixedArgs {
   double2* out_f;
   int64_t blk0;
   int32_t exit_trigger;  // may (in a launch: does) a pass let the next one launch at its blocks' exit only
+  int32_t nsm;           // SMs of the device
   int32_t uniform_v;  // every particle's V^ is exactly 1 (pass A leaves the V^ gathers out)
 };
 

@@ -1241,7 +1241,7 @@ static void (*pass_a_kernel(const MixedArgs& a, bool breaking))(MixedArgs) {
 // 14.7).  Up to two per SM both passes' blocks have their places at once (260 x 260 8.7 us; at the
 // exit 9.4), and a longer pass evens itself out (1M 82 us; 83.6).  Members of a batch, whose passes
 // run beside one another, let go at their start (16 plates of 67 .. 393 a side: 0.7 % of the call).
-constexpr int64_t kExitFrom = 2 * 152, kExitTo = 3 * 152;
+constexpr int64_t kExitFrom = 2, kExitTo = 3;
 
 static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_t sm, cudaStream_t s,
                             bool pdl = true) {
@@ -1257,7 +1257,8 @@ static void launch_pass_pdl(void (*kernel)(MixedArgs), const MixedArgs& a, size_
   lc.attrs = at;
   lc.numAttrs = pdl ? 1 : 0;
   MixedArgs b = a;
-  b.exit_trigger = a.exit_trigger && a.nblocks - a.blk0 > kExitFrom && a.nblocks - a.blk0 <= kExitTo;
+  const int64_t blocks = a.nblocks - a.blk0;
+  b.exit_trigger = a.exit_trigger && blocks > kExitFrom * a.nsm && blocks <= kExitTo * a.nsm;
   cudaLaunchKernelEx(&lc, kernel, b);
 }
 
