@@ -2152,8 +2152,9 @@ int pd_batch_create(int32_t device, int32_t precision, pd_batch** out) {
   if (!b) return PD_ERR_CAPACITY;
   b->device = device;
   b->precision = precision;
-  // every member's own step graph, concurrently (256-plate batch, ms per step: mixed 1.40 against
-  // 1.79 for the phase kernels and 1.89 for the persistent kernel; FP64 10.6 against 11.4 / 11.5)
+  // every member's own step graph, concurrently (256-plate batch, ms per step, bonds intact .. breaking:
+  // mixed 1.25 .. 1.38 against 1.64 for the phase kernels and 1.70 .. 1.78 for the persistent kernel;
+  // FP64 10.4 against 11.1 / 11.2)
   b->cfg.persistent = 2;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);

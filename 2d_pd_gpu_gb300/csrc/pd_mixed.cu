@@ -305,6 +305,11 @@ __global__ void __launch_bounds__(kBlock) k_drift_mixed(MixedArgs a) {
 // Slots per group of the walks (1M-particle plate, breaking: pass A 2, 3, 4
 // 51.5, 51.6, 50.9 us; 4M: 166, 163, 159; pass B 2, 4, 7: 49.9, 47.5, 53.5).
 constexpr int kWalkA = 4, kWalkB = 4;
+// Pass A of a batch's kernels, whose arguments lie in shared memory: three, and two where a
+// block is not staged (256 plates of 50 .. 400 a side with graded volumes, ms per step, phase
+// kernels: 4 and 4 slots 1.660, 4 and 1 1.648, 3 and 2 1.645, 2 and 1 1.679; persistent: 4 and 4 1.733,
+// 3 and 2 1.711).
+constexpr int kWalkABatch = 3, kWalkABatchUnstaged = 2;
 
 // Neighbour data gathered by the two passes.
 struct NbA {
@@ -335,7 +340,8 @@ __device__ __forceinline__ PreA load_a(const MixedArgs& a, int64_t p) {
 // out, which changes no result -- x * 1 and fma(1, x, y) are exact.
 // live: the lane has a particle (the whole warp calls it); spare: 512 B of the
 // warp's shared memory for the end of the walk.
-template <bool BREAK, bool UV, typename Idx, typename Gather>
+// W: slots per group of the walk.
+template <bool BREAK, bool UV, int W, typename Idx, typename Gather>
 __device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, bool live, const PreA& pre, int w, int64_t s0,
                                             Idx idx, Gather gather, float4* spare) {
   const float4 ui = pre.ui, xi = pre.xi;
@@ -399,7 +405,7 @@ __device__ __forceinline__ void pass_a_core(const MixedArgs& a, int64_t p, bool 
   // bonds breaking, of which ~4 us is the warp's K^-1 update)
   if (live) {
     int k = 0;
-    for (; k + kWalkA <= w; k += kWalkA) bonds(k, std::integral_constant<int, kWalkA>{});
+    for (; k + W <= w; k += W) bonds(k, std::integral_constant<int, W>{});
     for (; k < w; ++k) bonds(k, std::integral_constant<int, 1>{});
     a.hgs[p] = make_float2(2.f * a.k_hg * A.x, 2.f * a.k_hg * A.y);
   }
@@ -612,10 +618,14 @@ __device__ __forceinline__ void for_halo(const int32_t* H, int hn, int (&g)[kHal
 
 // Pass A of visiting block blk (kHaloBlock / 32 chunks) of plate a.  Every
 // thread of the kHaloBlock-thread block calls it; sm = the pass's dynamic
-// shared memory.  False if a staged copy timed out.  PDL: the pass may start
-// before the previous one has finished; until grid_dep_wait() it reads only
-// the visit record and the first halo ids, which no step writes.
-template <bool BREAK, bool PDL = false, bool UV = false>
+// shared memory.  False if a staged copy timed out.  PDL (not kNoPdl): the pass may
+// start before the previous one has finished; until grid_dep_wait() it reads only
+// the visit record and the first halo ids, which no step writes.  A batch's phase
+// kernels (kMember) let the next one go at once, without a look at exit_trigger (256
+// plates, 1.684 -> 1.660 ms per step).
+enum Pdl { kNoPdl, kAlone, kMember };
+
+template <bool BREAK, bool UV, Pdl PDL>
 __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, unsigned char* sm, uint64_t* bars) {
   int64_t chunk = 0, base = 0;
   int w = 0, nlive = 0;
@@ -628,7 +638,7 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
   if (PDL) {
     if (hn >= 0) halo_ids(a.halo + blk * a.halo_cap, hn, 0, g);
     grid_dep_wait();
-    if (!a.exit_trigger) grid_dep_launch();
+    if (PDL == kMember || !a.exit_trigger) grid_dep_launch();
   }
   PreA pre{};
   if (live) pre = load_a(a, p);  // in flight during the staging below
@@ -638,8 +648,8 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
     if (w > 0 && lane == 0) stage_issue(mine, a.nbr + base, (uint32_t)w * 128u, &bars[warp]);
     __syncwarp();
     if (!warp_stage_done(a, &bars[warp], w)) return false;
-    pass_a_core<BREAK, UV>(a, p, live, pre, w, base + lane, SharedIdx{mine, lane}, GatherA{&a},
-                           reinterpret_cast<float4*>(mine));
+    pass_a_core<BREAK, UV, PDL == kAlone ? kWalkA : kWalkABatchUnstaged>(
+        a, p, live, pre, w, base + lane, SharedIdx{mine, lane}, GatherA{&a}, reinterpret_cast<float4*>(mine));
     return true;
   }
   const HaloSmem h = halo_smem(a, sm);
@@ -658,15 +668,16 @@ __device__ __forceinline__ bool pass_a_block(const MixedArgs& a, int64_t blk, un
   const float4* q0 = h.q0;
   const float4* q1 = h.q1;
   const float* vh = h.vh;
-  pass_a_core<BREAK, UV>(a, p, live, pre, w, base + lane, SharedHaloIdx{h.li + warp * a.wmax * 32, lane},
-                     [=](int64_t l) { return NbA{q0[l], q1[l], UV ? 1.f : vh[l]}; },
-                         reinterpret_cast<float4*>(h.li + warp * a.wmax * 32));
+  uint16_t* mine = h.li + warp * a.wmax * 32;
+  pass_a_core<BREAK, UV, PDL == kAlone ? kWalkA : kWalkABatch>(
+      a, p, live, pre, w, base + lane, SharedHaloIdx{mine, lane},
+      [=](int64_t l) { return NbA{q0[l], q1[l], UV ? 1.f : vh[l]}; }, reinterpret_cast<float4*>(mine));
   return true;
 }
 
 // Pass B (+ the next drift when DRIFT, or the export when EXPORT) of
 // visiting block blk of plate a.  PDL: as for pass A.
-template <bool DRIFT, bool PDL = false, bool EXPORT = false>
+template <bool DRIFT, Pdl PDL, bool EXPORT = false>
 __device__ __forceinline__ bool pass_b_block(const MixedArgs& a, int64_t blk, unsigned char* sm, uint64_t* bars) {
   int64_t chunk = 0, base = 0;
   int w = 0, nlive = 0;
@@ -679,7 +690,7 @@ __device__ __forceinline__ bool pass_b_block(const MixedArgs& a, int64_t blk, un
   if (PDL) {
     if (hn >= 0) halo_ids(a.halo + blk * a.halo_cap, hn, 0, g);
     grid_dep_wait();
-    if (!a.exit_trigger) grid_dep_launch();
+    if (PDL == kMember || !a.exit_trigger) grid_dep_launch();
   }
   PreB pre{};
   if (live) pre = load_b<DRIFT, EXPORT>(a, p);  // in flight during the staging below
@@ -729,14 +740,14 @@ template <bool BREAK, bool UV>
 __global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock) k_pass_a_mixed(MixedArgs a) {  // <= 64 registers
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bars[kHaloBlock / 32];
-  pass_a_block<BREAK, true, UV>(a, a.blk0 + blockIdx.x, sm, bars);
+  pass_a_block<BREAK, UV, kAlone>(a, a.blk0 + blockIdx.x, sm, bars);
 }
 
 template <bool DRIFT>
 __global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock) k_pass_b_mixed(MixedArgs a) {  // <= 64 registers
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bars[kHaloBlock / 32];
-  pass_b_block<DRIFT, true>(a, a.blk0 + blockIdx.x, sm, bars);
+  pass_b_block<DRIFT, kAlone>(a, a.blk0 + blockIdx.x, sm, bars);
 }
 
 // The last pass B of pd_step_host: no drift, the new state written by
@@ -744,7 +755,7 @@ __global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock) k_pass_b_mixed(
 __global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock) k_pass_b_mixed_export(MixedArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bars[kHaloBlock / 32];
-  pass_b_block<false, true, true>(a, a.blk0 + blockIdx.x, sm, bars);
+  pass_b_block<false, kAlone, true>(a, a.blk0 + blockIdx.x, sm, bars);
 }
 
 // pd_step_host's import: the positions of visiting blocks blk0 .. blk1 - 1
@@ -1014,6 +1025,7 @@ __device__ __forceinline__ bool batch_phase_mixed(const MixedArgs* __restrict__ 
                                                   const BatchTile* __restrict__ tiles, int ntiles, int phase_rt,
                                                   unsigned char* sm, uint64_t* bars) {
   const int phase = PHASE < 0 ? phase_rt : PHASE;
+  constexpr Pdl kPdl = PHASE < 0 ? kNoPdl : kMember;
   bool ok = true;
   // the tile's plate arguments, copied to shared memory once per tile (the block code
   // reads them field by field; 2 % on the 256-plate batch)
@@ -1032,20 +1044,21 @@ __device__ __forceinline__ bool batch_phase_mixed(const MixedArgs* __restrict__ 
     if (phase == 0)
       drift_block(p, T.first);
     else if (phase == 1)  // the breaking pass also serves plates without breaking (their s2 is +inf)
-      ok = pass_a_block<true, (PHASE > 0)>(p, T.first, sm, bars);
+      ok = pass_a_block<true, false, kPdl>(p, T.first, sm, bars);
     else if (phase == 2)
-      ok = pass_b_block<true, (PHASE > 0)>(p, T.first, sm, bars);
+      ok = pass_b_block<true, kPdl>(p, T.first, sm, bars);
     else
-      ok = pass_b_block<false, (PHASE > 0)>(p, T.first, sm, bars);
+      ok = pass_b_block<false, kPdl>(p, T.first, sm, bars);
     ok = __syncthreads_and(ok);
   }
   return ok;
 }
 
-__global__ void __launch_bounds__(kHaloBlock) k_batch_persistent_mixed(const MixedArgs* __restrict__ plates,
-                                                                   const BatchTile* __restrict__ tiles, int ntiles,
-                                                                   int nsteps, GridBarrier* bar,
-                                                                   const BarrierLimits lim) {
+// Four blocks per SM, as the single-plate passes (left to itself the compiler takes 80 registers,
+// three blocks: 256 plates, 1.90 ms per step against 1.71).
+__global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock)
+    k_batch_persistent_mixed(const MixedArgs* __restrict__ plates, const BatchTile* __restrict__ tiles, int ntiles,
+                             int nsteps, GridBarrier* bar, const BarrierLimits lim) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bars[kHaloBlock / 32];
   const unsigned nb = gridDim.x;
@@ -1061,11 +1074,9 @@ __global__ void __launch_bounds__(kHaloBlock) k_batch_persistent_mixed(const Mix
   if (!ok && threadIdx.x == 0) atomicExch(&bar->err, 1);  // releases the other blocks' barrier waits
 }
 
-// registers as the single-plate passes: pass A 80 (3 blocks / SM), pass B 64 (4)
 template <int PHASE>
-__global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock)
-    k_batch_phase_mixed(const MixedArgs* __restrict__ plates,
-                                                              const BatchTile* __restrict__ tiles, int ntiles) {
+__global__ void __launch_bounds__(kHaloBlock, 1024 / kHaloBlock)  // as the single-plate passes
+    k_batch_phase_mixed(const MixedArgs* __restrict__ plates, const BatchTile* __restrict__ tiles, int ntiles) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint64_t bars[kHaloBlock / 32];
   batch_phase_mixed<PHASE>(plates, tiles, ntiles, PHASE, sm, bars);
