@@ -1752,6 +1752,11 @@ static int small_host_step(pd_ctx* c, int32_t nsteps, const double2* const in[3]
   cudaStream_t s = c->stream;
   const bool brk = c->p.s_c > 0.0;
   Launcher L(c);
+  cudaGraphExec_t inner = nullptr;
+  if (nsteps > kInnerSteps) {  // before anything is launched: a failure leaves the state as it was
+    const int rc = inner_graph(c, &inner);
+    if (rc != PD_OK) return rc;
+  }
   if (mixed(c)) {
     pd::launch_import_drift_mixed(L.m, 0, L.m.nblocks, in[0], in[1], in[2], s);
   } else {
@@ -1762,12 +1767,7 @@ static int small_host_step(pd_ctx* c, int32_t nsteps, const double2* const in[3]
     pd::launch_drift_fp64(z, s);
   }
   int32_t left = nsteps - 1;
-  for (; left >= kInnerSteps; left -= kInnerSteps) {
-    cudaGraphExec_t ge = nullptr;
-    const int rc = inner_graph(c, &ge);
-    if (rc != PD_OK) return rc;
-    PD_CK(c, cudaGraphLaunch(ge, s));
-  }
+  for (; left >= kInnerSteps; left -= kInnerSteps) PD_CK(c, cudaGraphLaunch(inner, s));
   for (; left > 0; --left) {
     L.pass_a(s);
     L.pass_b(true, s);
