@@ -1332,10 +1332,11 @@ int pd_checkpoint_load(pd_ctx* c, const void* buf, int64_t bytes) {
 // (slabs, multiples of 32), the first and the last ones short, so the first pass A
 // starts after a few microseconds of copying, the copies stay ahead of it, and the
 // slabs whose pass B and write-back end the call are brief.  From kFineSlabsFrom
-// particles on the even slabs between them hold about 62,000 particles each: fewer,
+// particles on the even slabs between them hold about 62,000 particles each, up to
+// kEvenMax of them (a plate of more than 1M particles has larger ones): fewer particles,
 // and their passes A leave SMs idle; more, and less of a slab's copies and write-back
 // runs under other slabs' passes (us per one-step call, 1M particles: 8 slabs 864,
-// 11 818, 14 806, 16 797, 19 790, 20 788).  Below, 11 slabs: more of them only cost
+// 11 818, 14 806, 16 797, 19 790, 20 788; 2M, 19 slabs 1512, 11 1566).  Below, 11 slabs: more of them only cost
 // launches (us: 360,000 particles: 11 slabs 347, 14 348, 19 356; 624,000: 11 slabs
 // 537, 14 545; 810,000: 11 slabs 675, 16 665).
 // slab_need[k] / slab_low[k] = the last / first slab holding a neighbour of
@@ -1717,7 +1718,10 @@ static cudaError_t enqueue_host_step_mixed(pd_ctx* c, int32_t nsteps, const doub
 // and write the page-locked buffers themselves, on one stream.  Per call, pipeline
 // against one stream, us: FP64, one step 100 x 100 213 / 65, 450 x 450 248 / 238,
 // 500 x 500 278 / 285, 1000 x 1000 814 / 974; mixed, one step 203 x 101 154 / 65,
-// 851 x 851 483 / 445, 1000 x 1000 537 / 554.
+// 851 x 851 483 / 445, 1000 x 1000 537 / 554.  Longer calls export after their last
+// step either way, and the one stream hands its passes over programmatically: calls of 2,
+// 4, 16 and 40 steps gain too (FP64 468 x 468 460 / 392, 803 / 699, 2856 / 2537, 6950 /
+// 6198; mixed 945 x 945 689 / 612, 846 / 761, 1772 / 1650, 3625 / 3419).
 constexpr int64_t kPipelineFrom = 220000, kPipelineFromMixed = 900000;
 
 // The graph of kInnerSteps steps between an import and the last step: pass A,

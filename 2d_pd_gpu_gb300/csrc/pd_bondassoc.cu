@@ -16,10 +16,12 @@
 //
 // The mode breaks no bond, and the weights depend on the reference geometry
 // and the parameters only, so what does not involve the displacements is
-// formed once, at set-up and on every parameter change, by the set-up form of
-// pass A (k_ba_pass_a<true>, after k_ba_bonds): per slot |xi|, 1/|xi|,
-// exp(+-n1 |xi| / l) and K_b^-1 with its det-guard flag; per particle, 1 / V_h
-// and, with <= 32 bonds, its weight matrix.
+// formed once, at set-up, on every parameter change and when a reset or a restore
+// changes the mask, by the set-up form of pass A (k_ba_pass_a<true>, after
+// k_ba_bonds): per slot |xi|, 1/|xi|, exp(+-n1 |xi| / l) and K_b^-1 with its
+// det-guard flag; per particle, 1 / V_h and, with <= 32 bonds, its weight matrix
+// (8 KB; where that would take more than a quarter of the free memory, its lower
+// triangle; where that does not fit, nothing: the weights are evaluated).
 //
 // Pass A runs one warp per particle and one lane per bond (families <= 64
 // bonds, two per lane): the family's bond data is staged in shared memory,
@@ -27,8 +29,9 @@
 // the weight matrix and forms V_q P_q, and, once every P_b is in shared memory,
 // lane j sums T_ij over b: 8 FP64 fma per ordered pair of bonds.  Where no family
 // exceeds 32 bonds the column stays in the lane's registers (k_ba_pass_a_small);
-// else the matrix is loaded into shared memory (k_ba_pass_a<false>).  A family of more than 32 bonds evaluates each lane's
-// weight row inside its D_q loop and keeps the rows of the first 32 bonds.
+// else the matrix is loaded into shared memory (k_ba_pass_a<false>).  A family of
+// more than 32 bonds evaluates each lane's weight row inside its D_q loop and keeps
+// the rows of the first 32 bonds.
 // The weight matrix is symmetric bit for bit (its products commute, and the
 // exponential factor is ordered by the two lengths), so only its lower
 // triangle is evaluated, spread over all 32 lanes.  The weight is evaluated in

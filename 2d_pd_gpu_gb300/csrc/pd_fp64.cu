@@ -2,10 +2,10 @@
 // only fused multiply-adds are the explicit fma() calls, written in the same
 // places as the oracle's restatement, so results are bit-identical to it.
 //
-// One thread per particle, bonds walked in family order through the SELL-32
-// layout (every slot load of a warp is one coalesced line).  Per-particle sums
-// are sequential in family order, with no atomics, so results are
-// deterministic and independent of the launch shape.
+// Two threads per particle, one per component, bonds walked in family order
+// through the SELL-32 layout (a warp's load of a slot is half a coalesced line).
+// Per-particle sums are sequential in family order, with no atomics, so results
+// are deterministic and independent of the launch shape.
 //
 // Reference correspondence (src/main_seq.cpp):
 //   k_drift / pass B tail : applyVelocityBC :28-36, updatePositions :386-393,
@@ -17,8 +17,10 @@
 //                           f_i = sum_j V_j (S_i + S_j) xi_ij (= T_ij - T_ji)
 // FP64 operations per bond: pass A 11 (d 2, stretch test 5, D 4) + 2 with the
 // zero-energy-mode penalty (sum V_j d), pass B 4.  The stretch test runs in
-// FP64 only for bonds within ~1e-6 of the limit (stretch_fp32 proves its
-// outcome for the others), so pass A costs 8 FP64 operations per bond.
+// FP64 only where stretch_fp32 cannot prove its outcome: about as near to the
+// limit s2 |xi|^2 as the larger of 1e-6 s2 |xi|^2 and 2.4e-7 (|u_i| + |u_j|) |xi|
+// (on a plate that has moved by 30 |xi|, at s_c = 5e-4: 1.4 % of the limit).  For
+// nearly every bond pass A costs 8 FP64 operations.
 #include "pd_internal.h"
 #include "pd_walk.cuh"
 
@@ -338,7 +340,7 @@ __device__ __forceinline__ int test_bonds(const Fp64Args& a, int64_t i, int h, i
 }
 
 // From this many particles (of the plate) on, pass A tests a particle's bonds before it sums them:
-// the sums then need 72 registers instead of 96 and no branch, and other warps' sums keep the FP64
+// the sums then need 80 registers instead of 96 and no branch, and other warps' sums keep the FP64
 // pipe busy under the tests (step with bonds breaking, us, 500 x 500 particles 176.7 -> 175.9,
 // 800 x 800 441 -> 435, 1M 683.5 -> 672, 2M 1356 -> 1329).  A smaller plate waits for the tests
 // (400 x 400 117.5 -> 118.1, 100 x 100 15.3 -> 15.9).  Where fewer than 3/4 of a warp's slots hold

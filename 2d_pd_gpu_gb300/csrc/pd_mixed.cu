@@ -136,21 +136,21 @@ constexpr int kManyLost = 14;
 __device__ __noinline__ void kinv_update_mixed_lanes(const MixedArgs& a, int64_t p, int64_t s0, int w, int newly,
                                                      const float4* D) {
   const int lane = threadIdx.x & 31;
-    bool bad = false;
-    if (newly > 0) {
-      const int64_t i = a.member[p];
-      const int32_t broken = a.broken[i] + newly;
-      a.broken[i] = broken;
-      a.damage[i] = (double)broken / (double)a.fam[i];
-      bad = kinv_update_mixed(a, i, p, s0, w);
-      const float4 d = D[lane];
-      a.ws[p] = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, f2(d.x, d.y), f2(d.z, d.w), a.geo[p]);
-    }
-    const int all = __reduce_add_sync(0xffffffffu, newly), nbad = __popc(__ballot_sync(0xffffffffu, bad));
-    if (lane == 0) {
-      atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)all);
-      if (nbad) atomicAdd(a.counters + CNT_SINGULAR, (unsigned long long)nbad);
-    }
+  bool bad = false;
+  if (newly > 0) {
+    const int64_t i = a.member[p];
+    const int32_t broken = a.broken[i] + newly;
+    a.broken[i] = broken;
+    a.damage[i] = (double)broken / (double)a.fam[i];
+    bad = kinv_update_mixed(a, i, p, s0, w);
+    const float4 d = D[lane];
+    a.ws[p] = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : w_of(a, f2(d.x, d.y), f2(d.z, d.w), a.geo[p]);
+  }
+  const int all = __reduce_add_sync(0xffffffffu, newly), nbad = __popc(__ballot_sync(0xffffffffu, bad));
+  if (lane == 0) {
+    atomicAdd(a.counters + CNT_BROKEN, (unsigned long long)all);
+    if (nbad) atomicAdd(a.counters + CNT_SINGULAR, (unsigned long long)nbad);
+  }
 }
 
 // Pass A's update of the particles that lost bonds (newly > 0 in their lane, p

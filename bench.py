@@ -180,7 +180,7 @@ DRAM_BYTES_PER_BOND = {"fp64": {"pass_a": 308.19e6 / 10031592, "pass_b": 246.97e
 
 def fp64_ops(n, nb):
     """FP64 operations per step of the FP64 form: pass A 8 per bond (d 2, D 4,
-    penalty sum 2; the stretch test is certified in FP32 for nearly all bonds)
+    penalty sum 2; the stretch test is decided in FP32 for nearly all bonds)
     + ~40 per particle, pass B 4 per bond + ~35 per particle."""
     return 12.0 * nb + 75.0 * n
 
