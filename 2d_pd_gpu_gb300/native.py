@@ -368,7 +368,8 @@ class Context:
     # -- stepping
     def step_host(self, nsteps, u, v, f, u_out=None, v_out=None, f_out=None):
         """pd_step_host: u, v, f ([n][2], page-locked: PinnedArray.array) in,
-        the new state written to the *_out buffers (default: in place)."""
+        the new state written to the *_out buffers (default: in place).  Arrays
+        that begin on 16 bytes are read and written directly, others by copies."""
         u_out = u if u_out is None else u_out
         v_out = v if v_out is None else v_out
         f_out = f if f_out is None else f_out
